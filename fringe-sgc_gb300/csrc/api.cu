@@ -119,10 +119,9 @@ int ensure_slots(fsgc_ctx* c, int n) {
   cudaStreamSynchronize(c->stream);
   cudaFree(c->d_slots);
   cudaFreeHost(c->h_slots);
-  cudaFree(c->d_member);
-  cudaFreeHost(c->h_member);
   c->d_slots = nullptr;
   c->h_slots = nullptr;
+  c->slot_cap = 0;
   CK(cudaMalloc((void**)&c->d_slots, sizeof(u64) * (size_t)cap), "slot allocation");
   CK(cudaMallocHost((void**)&c->h_slots, sizeof(u64) * (size_t)cap), "slot allocation");
   c->slot_cap = cap;

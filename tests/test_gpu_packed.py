@@ -58,3 +58,21 @@ def test_packed_rejects_crossing_edges(ctx):
     st = fsgc.lib().fsgc_graph_from_packed_csr(ctx.ptr, g.n, g.m, g.nindex.ctypes.data, g.nlist.ctypes.data, 2,
                                                vstart.ctypes.data, C.byref(gid))
     assert st != 0
+
+
+def test_packed_counts_survive_a_larger_batch(ctx):
+    """A batch that grows the context's result slots leaves the members' slots
+    of earlier packed counts alone."""
+    members = [fsgc.gen_er(60, 200, k) for k in range(5)]
+    pid = ctx.upload_packed(members)
+    gid = ctx.upload(members[0])
+    mo = fsgc.preprocess(*EXTRA["tailed_triangle_1"])
+    try:
+        want = [r.raw_total for r in ctx.count_packed(pid, mo)]
+        n = 2000
+        assert len({r.raw_total for r in ctx.count_batch([(gid, mo)] * n)}) == 1
+        assert [r.raw_total for r in ctx.count_packed(pid, mo)] == want
+        assert len(set(want)) > 1
+    finally:
+        ctx.release(pid)
+        ctx.release(gid)
