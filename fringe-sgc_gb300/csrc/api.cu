@@ -108,6 +108,13 @@ void free_graph(DevGraph* g) {
   cudaFree(g->ctab_id);
   cudaFree(g->ctab_rows);
   cudaFree(g->ctab_pos);
+  cudaFree(g->roff);
+  cudaFree(g->radj);
+  cudaFree(g->rdeg);
+  cudaFree(g->oid);
+  cudaFree(g->rrev);
+  cudaFree(g->radj16);
+  cudaFree(g->rtab);
   cudaFree(g->comp);
   cudaFree(g->comp_relabel);
   delete g;
