@@ -108,6 +108,7 @@ void free_graph(DevGraph* g) {
   cudaFree(g->ctab_id);
   cudaFree(g->ctab_rows);
   cudaFree(g->ctab_pos);
+  cudaFree(g->wide);
   cudaFree(g->roff);
   cudaFree(g->radj);
   cudaFree(g->rdeg);

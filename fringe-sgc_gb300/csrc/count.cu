@@ -8,13 +8,8 @@
 //   vertex core   one pass over the degrees;
 //   edge core     one pass over oriented edges, common-neighbour counts taken
 //                 from the loader's per-edge triangle supports;
-//   triangle core one block per lowest vertex a builds bitmap rows
-//                 N(a) & N(b_i) over the positions of N(a): the triangles are
-//                 the set bits, pairwise overlaps come from the supports and
-//                 the triple overlap is a popcount of two rows (the 4-clique
-//                 modes, and graphs whose out-lists would not fit in shared
-//                 memory, enumerate triangles on the oriented graph and take
-//                 the triple overlap by a warp-cooperative intersection);
+//   triangle core bitmap rows per lowest vertex (triangle.cu); here only for
+//                 out-degrees beyond its tables;
 //   wedge core    (centre without fringes) aggregated per endpoint pair: the
 //                 reference evaluates the same formula once per centre, and
 //                 the formula does not depend on the centre, so each pair is
@@ -38,14 +33,10 @@ namespace fsgc {
 void upload_div_magic() {
   upload_div_table();
   upload_div_magic_wedge();
+  upload_div_magic_triangle();
 }
 
 namespace {
-
-struct Rot3 {
-  int fr[6][8];
-  int count;
-};
 
 // ------------------------------------------------------------- vertex core
 template <class A>
@@ -162,16 +153,8 @@ __global__ void edge_set_kernel(GView g, EdgeSet p) {
 }
 
 // ------------------------------------------------------------- triangle core
-struct TriParams {
-  int sum1, sum2, sum3;
-  int mode;   // 0 general, 1 4-clique, 2 tailed 4-clique
-  int tails;
-  int relabel;  // roles by (deg, id) order (1) or by id (0)
-  int kmax;     // largest out-degree (bitmap kernel)
-  int stage;    // bitmap kernel: longest N(a) staged in shared memory (ints, multiple of 32)
-  int walk_ratio;  // bitmap kernel: walk N(b) when deg b <= walk_ratio * deg a
-  Rot3 rot;
-};
+// Graphs with out-degrees beyond triangle.cu's tables: triangles by merging
+// out-lists, triple overlaps by a warp-cooperative intersection.
 
 // Merge step over two sorted out-lists: advance (i,k) to the next common element.
 __device__ __forceinline__ bool next_common(const int* A, int la, const int* B, int lb, int& i, int& k) {
@@ -207,7 +190,7 @@ __device__ __forceinline__ long long tri_key(int x, int d, int relabel) {
 // One lane per oriented edge (a -> b); triangles a < b < c are found by merging
 // the out-lists.  Found triangles are served one at a time by the whole warp.
 template <class Ar>  // (A and B name out-lists below)
-__global__ void triangle_core_kernel(GView g, TriParams p, u64* __restrict__ slot) {
+__global__ void triangle_core_kernel(GView g, TrianglePattern p, u64* __restrict__ slot) {
   const int lane = threadIdx.x & 31;
   const long long me = g.m / 2;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -320,199 +303,6 @@ __global__ void triangle_core_kernel(GView g, TriParams p, u64* __restrict__ slo
     }
   }
   block_sum_to(acc, slot);
-}
-
-// Triangle core, general placements: one block per vertex a, handling every
-// triangle whose lowest (deg, id) vertex is a.  For each out-neighbour b_i of a
-// the block builds the bitmap M_i of N(a) & N(b_i) over the positions of N(a).
-// Then a pair (b_i, b_j) is a triangle iff bit pos(b_j) of M_i is set,
-// |N(a) & N(b_i)| = popc(M_i), and the triple overlap |N(a) & N(b_i) & N(b_j)|
-// = popc(M_i & M_j) -- a few word operations per triangle instead of an
-// intersection of full neighbour lists.
-//
-// N(a) is staged in shared memory by a bulk copy when it fits p.stage ints.  A
-// row then takes the cheaper of two ways: walk N(b_i) from global memory
-// (coalesced) and look each entry up in the staged N(a), building the row in
-// a per-warp shared buffer, when deg b_i <= p.walk_ratio * deg a; otherwise
-// test each entry of N(a) by a binary search of N(b_i) (one ballot per 32).
-constexpr int kTriThreads = 256;
-constexpr int kBulkWaitPolls = 1 << 22;  // bounded wait for a bulk copy
-
-// Triangle-core patterns of one pass: the bitmaps, roles and Venn sizes of a
-// triangle do not depend on the pattern, only the pruning thresholds and the
-// placement formulas do.  p.sum1 (the vertex gate) is the set's smallest.
-// Every launch today carries one pattern (see enqueue_count_set).
-constexpr int kTriFuse = 4;
-struct TriSet {
-  int np;
-  int sum1[kTriFuse], sum2[kTriFuse], sum3[kTriFuse];
-  Rot3 rot[kTriFuse];
-  u64* slot[kTriFuse];
-};
-
-template <int NP, class A>
-__global__ void __launch_bounds__(kTriThreads, 3) triangle_bitmap_kernel(GView g, TriParams p, TriSet ts,
-                                                                      int* __restrict__ queue,
-                                                                      unsigned* __restrict__ bits_all,
-                                                                      long long bits_per_block,
-                                                                      unsigned long long* __restrict__ err) {
-  extern __shared__ __align__(16) int s_dyn[];
-  __shared__ int s_a;
-  __shared__ __align__(8) unsigned long long s_bar;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  unsigned* bits = bits_all + (size_t)blockIdx.x * (size_t)bits_per_block;
-  const int kmax = p.kmax, stage = p.stage;
-  int* s_na = s_dyn;                              // staged N(a): stage + 4 ints (16-byte aligned)
-  unsigned* s_row = reinterpret_cast<unsigned*>(s_dyn + stage + 4);  // per warp: stage / 32 words
-  int* outl = s_dyn + stage + 4 + (stage >> 5) * (kTriThreads >> 5);  // out-neighbours of a
-  int* pos = outl + kmax;                         // their positions in N(a)
-  int* rowpop = outl + 2 * kmax;                  // |N(a) & N(b_i)|
-  unsigned parity = 0;
-  if (threadIdx.x == 0 && stage > 0) mbar_init(&s_bar, 1);
-  __syncthreads();
-  A acc[NP];
-#pragma unroll
-  for (int q = 0; q < NP; q++) acc[q] = A(0);
-  for (;;) {
-    if (threadIdx.x == 0) s_a = atomicAdd(queue, 1);
-    __syncthreads();
-    const int a = s_a;
-    if (a >= g.n) break;
-    const long long ob = g.ooff[a];
-    const int k = (int)(g.ooff[a + 1] - ob);
-    const int da = g.deg[a];
-    if (k >= 2 && da >= p.sum1) {
-      const int W = (da + 31) >> 5;
-      const long long abeg = g.off[a];
-      const bool staged = da <= stage;
-      const int* Na = g.adj + abeg;
-      if (staged) {
-        // the copy starts at the 16-byte boundary at or below N(a) (the list
-        // array is padded by 16 bytes, so the rounded-up end stays inside it)
-        const long long cbeg = abeg & ~3LL;
-        const int shift = (int)(abeg - cbeg);
-        if (threadIdx.x == 0) {
-          fence_proxy_async_smem();
-          const unsigned bytes = (unsigned)(((shift + da) * 4 + 15) & ~15);
-          bulk_copy_g2s(s_na, g.adj + cbeg, bytes, &s_bar);
-        }
-        const bool done = mbar_wait_bounded(&s_bar, parity, kBulkWaitPolls);
-        parity ^= 1u;
-        if (__syncthreads_or(!done)) {
-          // the copy did not complete: report it, give the copy one more
-          // bounded wait and leave (the count is void)
-          if (threadIdx.x == 0) atomicOr(err, 1ULL);
-          mbar_wait_bounded(&s_bar, parity ^ 1u, kBulkWaitPolls);
-          return;
-        }
-        Na = s_na + shift;
-      }
-      for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        const int b = g.oadj[ob + i];
-        outl[i] = b;
-        pos[i] = lower_bound_any(Na, da, b);  // Na may be the shared-memory stage
-        rowpop[i] = (int)g.osup[ob + i];  // |N(a) & N(b_i)| is the edge's support
-      }
-      // bitmaps: row i = N(a) & N(b_i), skipped when the edge closes no triangle
-      unsigned* wrow = s_row + warp * (stage >> 5);
-      for (int i = warp; i < k; i += nwarp) {
-        if (g.osup[ob + i] == 0) continue;
-        const int b = g.oadj[ob + i];
-        const int* Nb = g.adj + g.off[b];
-        const int db = g.deg[b];
-        unsigned* row = bits + (size_t)i * W;
-        if (staged && (long long)db <= (long long)p.walk_ratio * da) {
-          for (int w = lane; w < W; w += 32) wrow[w] = 0u;
-          __syncwarp();
-          // only N(b) entries inside [min N(a), max N(a)] can match
-          const int t0 = lower_bound_dev(Nb, db, Na[0]);
-          const int t1 = lower_bound_dev(Nb, db, Na[da - 1] + 1);
-          for (int t = t0 + lane; t < t1; t += 32) {
-            const int y = __ldg(Nb + t);
-            int lo = 0, hi = da;  // y's position in the staged N(a)
-            while (lo < hi) {
-              const int mid = (lo + hi) >> 1;
-              if (Na[mid] < y) lo = mid + 1;
-              else hi = mid;
-            }
-            if (lo < da && Na[lo] == y) atomicOr(&wrow[lo >> 5], 1u << (lo & 31));
-          }
-          __syncwarp();
-          for (int w = lane; w < W; w += 32) row[w] = wrow[w];
-          __syncwarp();
-        } else {
-          for (int w = 0; w < W; w++) {
-            const int x = w * 32 + lane;
-            const bool hit = (x < da) && bsearch_has(Nb, db, Na[x]);
-            const unsigned word = __ballot_sync(0xffffffffu, hit);
-            if (lane == 0) row[w] = word;
-          }
-        }
-      }
-      __syncthreads();
-      // pairs (i, j), i < j: warp per row, lanes over j
-      for (int i = warp; i < k - 1; i += nwarp) {
-        if (rowpop[i] == 0) continue;
-        const unsigned* Mi = bits + (size_t)i * W;
-        const int bi = outl[i], di = g.deg[bi];
-        for (int j = i + 1 + lane; j < k; j += 32) {
-          const int pj = pos[j];
-          if (!((Mi[pj >> 5] >> (pj & 31)) & 1u)) continue;
-          const int bj = outl[j], dj = g.deg[bj];
-          const unsigned* Mj = bits + (size_t)j * W;
-          int c123 = 0;
-          for (int w = 0; w < W; w++) c123 += __popc(Mi[w] & Mj[w]);
-          // support of edge (b_i, b_j): slot in the out-list of the lower one
-          const bool i_low = (di < dj) || (di == dj && bi < bj);
-          const int lo = i_low ? bi : bj, hi = i_low ? bj : bi;
-          const long long lb = g.ooff[lo];
-          const int sl = bsearch_pos(g.oadj + lb, (int)(g.ooff[lo + 1] - lb), hi);
-          const int s_ij = (int)g.osup[lb + sl];
-          // roles u (latest), v, w (earliest) in the reference's vertex order
-          const int xv[3] = {a, bi, bj};
-          const int dx[3] = {da, di, dj};
-          long long kx[3];
-          const int rl = relabel_of(g, p.relabel, a);
-          for (int t = 0; t < 3; t++) kx[t] = tri_key(xv[t], dx[t], rl);
-          int ord[3] = {0, 1, 2};
-          if (kx[ord[0]] < kx[ord[1]]) { int t = ord[0]; ord[0] = ord[1]; ord[1] = t; }
-          if (kx[ord[1]] < kx[ord[2]]) { int t = ord[1]; ord[1] = ord[2]; ord[2] = t; }
-          if (kx[ord[0]] < kx[ord[1]]) { int t = ord[0]; ord[0] = ord[1]; ord[1] = t; }
-          // pairwise overlaps by vertex slot: 0 = a, 1 = b_i, 2 = b_j
-          const int sup01 = rowpop[i], sup02 = rowpop[j], sup12 = s_ij;
-          auto sup = [&](int x, int y) {
-            const int s = x + y;  // 1 -> (0,1), 2 -> (0,2), 3 -> (1,2)
-            return s == 1 ? sup01 : (s == 2 ? sup02 : sup12);
-          };
-          const int iu = ord[0], iv = ord[1], iw = ord[2];
-          const int du = dx[iu], dv = dx[iv], dw = dx[iw];
-          const int p12 = sup(iu, iv), t13 = sup(iu, iw), t23 = sup(iv, iw);
-          const int c12 = p12 - (c123 + 1), c13 = t13 - (c123 + 1), c23 = t23 - (c123 + 1);
-          int venn[8];
-          venn[0] = 0;
-          venn[IU] = du - (c12 + c13 + (c123 + 2));
-          venn[IV] = dv - (c12 + c23 + (c123 + 2));
-          venn[IW] = dw - (c13 + c23 + (c123 + 2));
-          venn[IUV] = c12; venn[IUW] = c13; venn[IVW] = c23; venn[IUVW] = c123;
-#pragma unroll
-          for (int q = 0; q < NP; q++) {
-            if (q >= ts.np) break;
-            // the reference's pruning (init_wl_triangle, common3_triangle)
-            const int th1 = max(ts.sum1[q], ts.sum2[q] - du);
-            const int th2 = max(max(ts.sum1[q], ts.sum3[q] - du - dv), max(ts.sum2[q] - du, ts.sum2[q] - dv));
-            if (!((du >= ts.sum1[q]) && (dv >= th1) && (dw >= th2))) continue;
-            A t = A(0);
-            for (int r = 0; r < ts.rot[q].count; r++) t += fc3<A>(ts.rot[q].fr[r], venn);
-            credit(g, acc[q], t, a);
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < NP; q++)
-    if (q < ts.np) block_sum_to(acc[q], ts.slot[q]);
 }
 
 // ------------------------------------------------------------- wedge core
@@ -1447,6 +1237,8 @@ int ensure_chunk_table(DevGraph& G, cudaStream_t s, uint64_t* launches, u64* d_s
   return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
 
+}  // namespace
+
 // Stream-ordered, so that growing one stream's arena neither waits for nor
 // stalls work queued on other streams.
 int ensure_plain_scratch(Scratch& sc, size_t need, cudaStream_t s) {
@@ -1465,41 +1257,6 @@ int ensure_plain_scratch(Scratch& sc, size_t need, cudaStream_t s) {
   sc.gen++;
   return FSGC_OK;
 }
-
-// Triangle bitmap kernel geometry: rows of ceil(deg/32) words per out-neighbour
-// of the block's vertex, one arena of max_bitmap_words per block, at most 8 GiB;
-// three resident blocks per SM (the kernel is built for 80 registers a thread).
-void triangle_bitmap_geometry(const DevGraph& G, long long* per_block, int* blocks) {
-  *per_block = std::max(1LL, G.max_bitmap_words);
-  const size_t budget = (size_t)8 << 30;
-  *blocks = (int)std::max<size_t>(
-      1, std::min<size_t>((size_t)sm_count() * 3, budget / (sizeof(unsigned) * (size_t)*per_block)));
-}
-
-bool triangle_uses_bitmaps(const fsgc_matching_order&, const DevGraph& G, int mode) {
-  const size_t smem = (size_t)3 * sizeof(int) * (size_t)std::max(1LL, G.max_outdeg);
-  return mode == 0 && smem <= (size_t)96 * 1024 && G.m / 2 > 0;
-}
-
-// Bitmap kernel shared memory: the out-neighbour arrays (3 ints each), then as
-// long an N(a) stage as fits a 72 KB block (three blocks per SM): 4 bytes per
-// staged entry plus one row bit per warp, up to stage_max entries.  Returns the
-// stage length (a multiple of 32, or 0) and the block's dynamic shared memory.
-// The bitmap rows stay in the global arena: keeping the rows of small vertices
-// in a full 72 KB block made the 4-clique pattern of the RMAT-22 benchmark 58%
-// slower, most likely because the larger shared-memory carve-out leaves the
-// kernel's list reads a small L1.
-int triangle_stage(int kmax, int stage_max, size_t* smem) {
-  const long long fixed = 3LL * 4 * std::max(1, kmax);
-  const long long budget = 72LL * 1024 - fixed - 16;
-  long long stage = budget > 0 ? budget / (4 + (kTriThreads / 32) * 4 / 32) : 0;
-  stage = std::min<long long>(stage, std::min(8192, std::max(0, stage_max))) & ~31LL;
-  if (stage < 64) stage = 0;
-  *smem = (size_t)(4 * (stage + 4) + 4 * (stage / 32) * (kTriThreads / 32) + fixed);
-  return (int)stage;
-}
-
-}  // namespace
 
 // What a count of `mo` on `G` needs beyond the resident graph.  The shape
 // tests repeat enqueue_count's dispatch.
@@ -1542,11 +1299,11 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
   }
   const bool clique = (f[IUVW] == 1) && (f[IUV] + f[IUW] + f[IVW] == 0) &&
                       ((f[IU] == 0) + (f[IV] == 0) + (f[IW] == 0) >= 2);
-  if (triangle_uses_bitmaps(mo, G, clique ? 1 : 0)) {
-    long long per_block;
-    int blocks;
-    triangle_bitmap_geometry(G, &per_block, &blocks);
-    nd.scratch = sizeof(unsigned) * (size_t)per_block * (size_t)blocks;
+  if (!clique && triangle_by_tables(G)) {
+    // rows of vertices that do not fit in shared memory: at most three blocks'
+    // worth per SM and 8 GiB (an upper bound of what enqueue_triangle takes)
+    const size_t per_block = sizeof(unsigned) * (size_t)std::max(1LL, G.max_bitmap_words);
+    nd.scratch = per_block * std::max<size_t>(1, std::min<size_t>((size_t)sm_count() * 3, ((size_t)8 << 30) / per_block));
   }
   return nd;
 }
@@ -1639,34 +1396,6 @@ int launch_wedge_set(DevGraph& G, const GView& gv, const WedgeSet& ws0, cudaStre
     wedge_chunk_kernel<true, NP, A><<<blocks, kWThreads, smem, s>>>(gv, ws, q2, gcur, gpre, gs, tab);
     *launches += 1;
   }
-  return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
-}
-
-// The triangle bitmap kernel for a set of patterns (tp: shared fields, with
-// tp.sum1 the set's smallest vertex gate).
-template <int NP, class A>
-int launch_triangle_set(DevGraph& G, const GView& gv, TriParams tp, const TriSet& ts, cudaStream_t s,
-                        uint64_t* launches, DevWork& work) {
-  size_t smem = 0;
-  tp.kmax = (int)G.max_outdeg;
-  tp.stage = triangle_stage(tp.kmax, work.tune.triangle_stage_max, &smem);
-  tp.walk_ratio = std::max(0, work.tune.triangle_walk_ratio);
-  long long per_block;
-  int blocks;
-  triangle_bitmap_geometry(G, &per_block, &blocks);
-  const size_t need = sizeof(unsigned) * (size_t)per_block * (size_t)blocks;
-  int st = ensure_plain_scratch(work.tri, need, s);
-  if (st != FSGC_OK) return st;
-  int* queue = reinterpret_cast<int*>(work.small + 6);
-  cudaMemsetAsync(queue, 0, sizeof(int), s);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(triangle_bitmap_kernel<NP, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  triangle_bitmap_kernel<NP, A><<<blocks, kTriThreads, smem, s>>>(
-      gv, tp, ts, queue, reinterpret_cast<unsigned*>(work.tri.ptr), per_block,
-      reinterpret_cast<unsigned long long*>(work.small + kErrWord));
-  *launches += 1;
-  // the kernel's error bits (a bulk copy that never completed) for the caller
-  if (work.h_err) cudaMemcpyAsync(work.h_err, work.small + kErrWord, sizeof(u64), cudaMemcpyDeviceToHost, s);
   return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
 
@@ -1778,7 +1507,7 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
     const int min_u = f[IUVW] + f[IUV] + f[IUW] + f[IU];
     const int min_v = f[IUVW] + f[IUV] + f[IVW] + f[IV];
     const int min_w = f[IUVW] + f[IUW] + f[IVW] + f[IW];
-    TriParams tp;
+    TrianglePattern tp;
     tp.sum3 = min_u + min_v + min_w + 6;
     tp.sum2 = tp.sum3 - (std::max(std::max(min_u, min_v), min_w) + 2);
     tp.sum1 = std::min(std::min(min_u, min_v), min_w) + 2;
@@ -1787,20 +1516,11 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
     tp.tails = f[IU] + f[IV] + f[IW];
     tp.mode = clique ? (tp.tails == 0 ? 1 : 2) : 0;
     tp.relabel = G.tri_relabel ? 1 : 0;
-    tp.kmax = (int)G.max_outdeg;
     rotations3(f, false, tp.rot);
     if (me == 0) return FSGC_OK;
-    if (triangle_uses_bitmaps(mo, G, tp.mode)) {
-      TriSet ts;
-      memset(&ts, 0, sizeof(ts));
-      ts.np = 1;
-      ts.sum1[0] = tp.sum1; ts.sum2[0] = tp.sum2; ts.sum3[0] = tp.sum3;
-      ts.rot[0] = tp.rot;
-      ts.slot[0] = job.d_slot;
-      return launch_triangle_set<1, A>(G, gv, tp, ts, s, launches, work);
-    } else {
-      triangle_core_kernel<A><<<grid_for(me, TPB, 8), TPB, 0, s>>>(gv, tp, job.d_slot);
-    }
+    if (triangle_by_tables(G))
+      return enqueue_triangle(G, gv, tp, std::is_same<A, X128>::value, job.d_slot, s, launches, work);
+    triangle_core_kernel<A><<<grid_for(me, TPB, 8), TPB, 0, s>>>(gv, tp, job.d_slot);
     *launches += 1;
     return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
   }
@@ -1860,8 +1580,7 @@ int enqueue_count(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& wo
 // Many patterns on one graph: patterns whose kernels share their match
 // enumeration run as sets -- stars and tailed triangles in one vertex pass,
 // edge-core formulas in one pass over the oriented edges, fringe-free-centre
-// wedges over one set of centre counts, triangle cores over one set of
-// bitmaps -- and every other pattern as a count of its own.  Each job's
+// wedges together -- and every other pattern as a count of its own.  Each job's
 // result goes to its own slot; the values equal the single-pattern kernels'.
 int enqueue_count_set(std::vector<CountJob*>& jobs, cudaStream_t s, uint64_t* launches, DevWork& work) {
   if (jobs.empty()) return FSGC_OK;
@@ -1874,7 +1593,6 @@ int enqueue_count_set(std::vector<CountJob*>& jobs, cudaStream_t s, uint64_t* la
   std::vector<std::pair<CountJob*, std::pair<int, int>>> verts;  // (job, (tailed, t))
   std::vector<std::pair<CountJob*, EdgeParams>> edges;
   std::vector<std::pair<CountJob*, WedgeParams>> wedges;
-  std::vector<std::pair<CountJob*, TriParams>> tris;
   std::vector<CountJob*> single;
   for (CountJob* jp : jobs) {
     CountJob& job = *jp;
@@ -1913,24 +1631,6 @@ int enqueue_count_set(std::vector<CountJob*>& jobs, cudaStream_t s, uint64_t* la
           const int min_w = f[IUVW] + f[IUW] + f[IVW] + f[IW] + 1;
           job.core_type = FSGC_CORE_WEDGE;
           wedges.push_back({jp, WedgeParams{f[IV], f[IVW], f[IW], std::min(min_v, min_w), min_v + min_w}});
-          continue;
-        }
-      } else {
-        const int min_u = f[IUVW] + f[IUV] + f[IUW] + f[IU];
-        const int min_v = f[IUVW] + f[IUV] + f[IVW] + f[IV];
-        const int min_w = f[IUVW] + f[IUW] + f[IVW] + f[IW];
-        const bool clique = (f[IUVW] == 1) && (f[IUV] + f[IUW] + f[IVW] == 0) &&
-                            ((f[IU] == 0) + (f[IV] == 0) + (f[IW] == 0) >= 2);
-        if (!clique && triangle_uses_bitmaps(mo, G, 0)) {
-          TriParams tp;
-          memset(&tp, 0, sizeof(tp));
-          tp.sum3 = min_u + min_v + min_w + 6;
-          tp.sum2 = tp.sum3 - (std::max(std::max(min_u, min_v), min_w) + 2);
-          tp.sum1 = std::min(std::min(min_u, min_v), min_w) + 2;
-          tp.relabel = G.tri_relabel ? 1 : 0;
-          rotations3(f, false, tp.rot);
-          job.core_type = FSGC_CORE_TRIANGLE;
-          tris.push_back({jp, tp});
           continue;
         }
       }
@@ -1981,21 +1681,6 @@ int enqueue_count_set(std::vector<CountJob*>& jobs, cudaStream_t s, uint64_t* la
     }
     st = ws.np == 1 ? launch_wedge_set<1, u64>(G, gv, ws, s, launches, work)
                     : launch_wedge_set<kWedgeFuse, u64>(G, gv, ws, s, launches, work);
-    if (st != FSGC_OK) return st;
-  }
-  // Triangle-core patterns get one bitmap pass each.  A pass over four
-  // patterns shares the row build, but its kernel carries four inlined copies
-  // of fc3 and spills: six fringe-heavy triangle patterns on RMAT-20 took 31 s
-  // in passes of four and two against 20 s one by one.
-  for (const auto& t : tris) {
-    TriSet ts;
-    memset(&ts, 0, sizeof(ts));
-    const TriParams& tp = t.second;
-    ts.np = 1;
-    ts.sum1[0] = tp.sum1; ts.sum2[0] = tp.sum2; ts.sum3[0] = tp.sum3;
-    ts.rot[0] = tp.rot;
-    ts.slot[0] = t.first->d_slot;
-    st = launch_triangle_set<1, u64>(G, gv, tp, ts, s, launches, work);
     if (st != FSGC_OK) return st;
   }
   for (CountJob* jp : single) {

@@ -56,6 +56,7 @@ __host__ __device__ inline u64 nck_ref(int n, int k, const DivMagic* tab) {
   k = (k < n - k) ? k : n - k;
   if (k < 0) return 0;
   if (k == 0) return 1;
+  if (k == 2) return ((u64)n * (u64)(n - 1)) >> 1;  // below 2^62: the loop's value without its division
   u64 r = (u64)n;
   for (int i = 2; i <= k; i++) {
     r = r * (u64)(n + 1 - i);
@@ -129,56 +130,8 @@ __device__ __forceinline__ int lower_bound_dev(const int* __restrict__ a, int le
   return lo;
 }
 
-// number of elements < x in a[0..len) with plain loads: for lists that may sit
-// in shared memory (the __ldg searches above take global addresses only)
-__device__ __forceinline__ int lower_bound_any(const int* a, int len, int x) {
-  int lo = 0, hi = len;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (a[mid] < x) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// ----------------------------------------------------------------------------
-// Bulk copies from global to shared memory (cp.async.bulk, the Blackwell copy
-// engine without a tensor map), completed on an mbarrier.  Source and
-// destination must be 16-byte aligned and the size a multiple of 16; the
-// copies used here read this GPU's own memory and are never multicast.
+// 32-bit shared-memory address of a pointer into shared memory.
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// Orders this thread's earlier shared-memory accesses before later copies.
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// One thread: arm the barrier for `bytes` and start the copy.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-// Waits for the barrier's phase `parity` to complete, polling at most `limit`
-// times; false when it gave up.
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity, int limit) {
-  for (int i = 0; i < limit; i++) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
 
 // ----------------------------------------------------------------------------
 // Exact counts: unsigned 128-bit values that saturate at 2^128 - 1 (every bit
@@ -257,6 +210,13 @@ __host__ __device__ inline X128 nck_x(int n, int k) {
 }
 
 // ----------------------------------------------------------------------------
+// Block barrier for kernels whose warps may arrive with their lanes apart: the
+// form of barrier.sync without .aligned counts threads.  __syncthreads() (the
+// aligned form) counted such warps twice after long divergent loops, which let
+// the others through early.
+__device__ __forceinline__ void block_sync() { asm volatile("barrier.sync 0;" ::: "memory"); }
+
+// ----------------------------------------------------------------------------
 // Reductions: warp shuffle -> one shared-memory atomic per warp -> one global
 // atomic per block into the task's result slot (mod 2^64 addition).
 __device__ __forceinline__ u64 warp_sum_u64(u64 v) {
@@ -266,14 +226,14 @@ __device__ __forceinline__ u64 warp_sum_u64(u64 v) {
 }
 __device__ __forceinline__ int warp_sum_int(int v) { return __reduce_add_sync(0xffffffffu, v); }
 
-// Every thread of the block must call this (it contains __syncthreads).
+// Every thread of the block must call this (it contains barriers).
 __device__ __forceinline__ void block_sum_to(u64 v, u64* __restrict__ slot) {
   __shared__ u64 s_acc;
   if (threadIdx.x == 0) s_acc = 0;
-  __syncthreads();
+  block_sync();
   v = warp_sum_u64(v);
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(&s_acc, v);
-  __syncthreads();
+  block_sync();
   if (threadIdx.x == 0 && s_acc) atomicAdd(slot, s_acc);
 }
 
@@ -291,7 +251,7 @@ __device__ __forceinline__ void block_sum_to(X128 v, u64* __restrict__ slot) {
     v = v + w;
   }
   if (lane == 0) { s_part[warp][0] = v.lo; s_part[warp][1] = v.hi; }
-  __syncthreads();
+  block_sync();
   if (threadIdx.x == 0) {
     X128 t;
     for (int i = 0; i < (int)((blockDim.x + 31) >> 5); i++) t = t + X128(s_part[i][0], s_part[i][1]);
@@ -311,7 +271,7 @@ __device__ __forceinline__ void block_sum_to(X128 v, u64* __restrict__ slot) {
       }
     }
   }
-  __syncthreads();  // s_part is free again for a later call
+  block_sync();  // s_part is free again for a later call
 }
 
 }  // namespace fsgc

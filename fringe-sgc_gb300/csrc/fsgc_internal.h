@@ -49,6 +49,8 @@ struct DevGraph {
   unsigned* osup = nullptr;
   long long triangles = -1;
   long long max_outdeg = 0;        // largest oriented out-degree
+  int* wide = nullptr;             // vertices whose triangles take a wide block each (triangle_wide)
+  int nwide = 0;
   long long max_bitmap_words = 0;  // max over v of outdeg(v) * ceil(deg(v) / 32)
   u64* vtri2 = nullptr;  // lazily
   unsigned* esup = nullptr;  // lazily: per list entry (u, v), |N(u) & N(v)|
@@ -128,6 +130,7 @@ int ensure_vertex_triangles(DevGraph& g, cudaStream_t s, uint64_t* launches);
 int ensure_entry_supports(DevGraph& g, cudaStream_t s, uint64_t* launches);
 void upload_div_magic();
 void upload_div_magic_wedge();
+void upload_div_magic_triangle();
 int sm_count();
 
 struct CountJob {
@@ -142,6 +145,38 @@ struct CountJob {
   int per_member_div;    // packed graphs: divide each member's total by this on the host (1 = none)
   bool exact_count = false;  // exact 128-bit sums: d_slot holds (lo, hi, saturated); ordinary graphs only
 };
+
+// Fringe counts of a 3-vertex core's anchor sets, one row per rotation.
+struct Rot3 {
+  int fr[6][8];
+  int count;
+};
+
+// Whether no C(n, i), n <= maxdeg, i <= k, wraps in u64 before its division:
+// C(n, i) i <= n^i / (i-1)! < 2^63.  Sums of products of them may then be
+// regrouped mod 2^64.
+bool binomials_fit(int maxdeg, int k);
+
+// Triangle core (triangle.cu).
+struct TrianglePattern {
+  int sum1, sum2, sum3;  // pruning thresholds
+  int mode;              // 0 general, 1 4-clique, 2 tailed 4-clique
+  int tails;
+  int relabel;           // roles by (deg, id) order (1) or by id (0)
+  Rot3 rot;
+};
+// Vertices with `k` out-neighbours and rows over `lists` positions that need the
+// larger blocks: more row words or a larger table than a narrow block holds, or
+// more lists than its four warps should read.
+constexpr int kTriNarrowK = 256, kTriNarrowRows = 6400, kTriNarrowLists = 4096;
+__host__ __device__ inline bool triangle_wide(int k, int lists) {
+  return k > kTriNarrowK || lists > kTriNarrowLists || (long long)k * (((lists + 31) >> 5) | 1) > kTriNarrowRows;
+}
+bool triangle_by_tables(const DevGraph& G);  // out-degrees small enough for that path
+int enqueue_triangle(DevGraph& G, const GView& gv, const TrianglePattern& tp, bool exact, u64* slot, cudaStream_t s,
+                     uint64_t* launches, DevWork& work);
+// Grows a work arena, stream-ordered.
+int ensure_plain_scratch(Scratch& sc, size_t need, cudaStream_t s);
 
 // Wedge core with a fringe-free centre: fringes of the larger-id endpoint, of
 // both and of the other, and the endpoint degrees below which it counts nothing.

@@ -202,21 +202,32 @@ __global__ void triangle_support_kernel(GView g, unsigned* __restrict__ osup, u6
   block_sum_to(tot, tri_total);
 }
 
-// largest out-degree and largest out-degree * ceil(deg / 32) (bitmap rows)
+// Largest out-degree, largest out-degree * ceil(deg / 32) (bitmap rows) and the
+// number of vertices whose triangles take a wide block.
 __global__ void outdeg_stats_kernel(GView g, unsigned long long* __restrict__ stats) {
-  unsigned long long k1 = 0, k2 = 0;
+  unsigned long long k1 = 0, k2 = 0, wide = 0;
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += gridDim.x * blockDim.x) {
     const unsigned long long k = (unsigned long long)(g.ooff[v + 1] - g.ooff[v]);
     k1 = max(k1, k);
     k2 = max(k2, k * (unsigned long long)((g.deg[v] + 31) >> 5));
+    wide += k >= 2 && triangle_wide((int)k, g.deg[v]);
   }
   for (int o = 16; o > 0; o >>= 1) {
     k1 = max(k1, __shfl_down_sync(0xffffffffu, k1, o));
     k2 = max(k2, __shfl_down_sync(0xffffffffu, k2, o));
+    wide += __shfl_down_sync(0xffffffffu, wide, o);
   }
   if ((threadIdx.x & 31) == 0) {
     atomicMax(stats, k1);
     atomicMax(stats + 1, k2);
+    if (wide) atomicAdd(stats + 2, wide);
+  }
+}
+
+__global__ void wide_list_kernel(GView g, int* __restrict__ list, int* __restrict__ count) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += gridDim.x * blockDim.x) {
+    const int k = (int)(g.ooff[v + 1] - g.ooff[v]);
+    if (k >= 2 && triangle_wide(k, g.deg[v])) list[atomicAdd(count, 1)] = v;
   }
 }
 
@@ -324,11 +335,11 @@ int prepare_graph(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_u64) {
     *launches += 1;
   }
   u64* d_stats = d_u64 + 2;
-  FSGC_TRY(cudaMemsetAsync(d_stats, 0, 2 * sizeof(u64), s));
+  FSGC_TRY(cudaMemsetAsync(d_stats, 0, 4 * sizeof(u64), s));  // the last: the list's fill count
   outdeg_stats_kernel<<<grid_for(n, kTPB, 8), kTPB, 0, s>>>(v, d_stats);
   *launches += 1;
-  u64 stats[3] = {0, 0, 0};
-  FSGC_TRY(cudaMemcpyAsync(stats, d_tri, 3 * sizeof(u64), cudaMemcpyDeviceToHost, s));
+  u64 stats[4] = {0, 0, 0, 0};
+  FSGC_TRY(cudaMemcpyAsync(stats, d_tri, 4 * sizeof(u64), cudaMemcpyDeviceToHost, s));
   FSGC_TRY(cudaFreeAsync(odeg, s));
   FSGC_TRY(cudaFreeAsync(tiles, s));
   FSGC_TRY(cudaStreamSynchronize(s));
@@ -336,6 +347,14 @@ int prepare_graph(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_u64) {
   g.triangles = (long long)stats[0];
   g.max_outdeg = (long long)stats[1];
   g.max_bitmap_words = (long long)stats[2];
+  if (stats[3] > 0) {
+    FSGC_TRY(cudaMallocAsync((void**)&g.wide, sizeof(int) * (size_t)stats[3], s));
+    wide_list_kernel<<<grid_for(n, kTPB, 8), kTPB, 0, s>>>(v, g.wide, reinterpret_cast<int*>(d_stats + 3));
+    *launches += 1;
+    FSGC_TRY(cudaStreamSynchronize(s));
+    g.nwide = (int)stats[3];
+    g.bytes += sizeof(int) * (size_t)stats[3];
+  }
   // the reference relabels (and so orders triangle roles by degree) only for
   // n > 10000, n <= m/10 and maximum degree > 16
   g.tri_relabel = (n > 10000) && !((long long)n > g.m / 10) && (maxd > 16);

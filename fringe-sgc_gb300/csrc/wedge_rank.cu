@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
           s_p[warp] = pe + p;
           s_q[warp] = qe + q;
         }
-        __syncthreads();
+        block_sync();
         if (threadIdx.x == 0) {
           A ps = A(0), qs = A(0);
           for (int w = 0; w < kTPB / 32; w++) {
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
             qs += s_q[w];
           }
         }
-        __syncthreads();
+        block_sync();
         if (g.comp) {
           a2 = warp_sum_a(a2);
           if (lane == 0 && a2) slot_add(a2, g.comp_slots + g.comp[h]);
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
         }
       }
     }
-    __syncthreads();  // s_big is free again
+    block_sync();  // s_big is free again
   }
   warp_sum_to(total, slot);
 }
@@ -332,7 +332,7 @@ __device__ __forceinline__ void list_segments(RankSmem& S, int n, const int* st,
       S.warp_tmp[(2 + h) * kRW + warp] = es[h] + b;
     }
   }
-  __syncthreads();
+  block_sync();
   // lanes 0..15: long totals of one half's warps, lanes 16..31: short totals
   u64 cl = 0, cs = 0;
 #pragma unroll
@@ -374,7 +374,7 @@ __device__ __forceinline__ void list_segments(RankSmem& S, int n, const int* st,
     S.pre[nl] = (int)(unsigned)cl;
     S.pre[nl + 1 + (int)(cs >> 32)] = (int)(unsigned)cs;
   }
-  __syncthreads();
+  block_sync();
 }
 
 // index in [a, b) of the last prefix value <= e
@@ -804,12 +804,12 @@ __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constan
   int next = 0;  // thread 0: the item after this one, fetched while this one runs
   if (tid == 0) next = atomicAdd(queue, 1);
   for (;;) {
-    __syncthreads();
+    block_sync();
     if (tid == 0) {
       S.item = next;
       S.nlist = 0;
     }
-    __syncthreads();
+    block_sync();
     const int item = S.item;
     if (tid == 0) next = atomicAdd(queue, 1);
     if (item < heavy) {
@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constan
         if (block && lane == 0) S.list[atomicAdd(&S.nlist, 1)] = v;
       }
     }
-    __syncthreads();
+    block_sync();
     const int nlist = S.nlist;
     for (int li = 0; li < nlist; li++) {
       const int v = S.list[li];
@@ -905,7 +905,7 @@ __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constan
         S.centres = 0;
         S.last = -1;
       }
-      __syncthreads();
+      block_sync();
       {
         unsigned long long sum = 0;
         int some = 0, last = -1;
@@ -931,7 +931,7 @@ __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constan
           atomicMax(&S.last, last);
         }
       }
-      __syncthreads();
+      block_sync();
       const unsigned long long wedges = S.wedges;
       const int top = S.last;  // the largest w any centre reaches
       if (S.centres >= 2) {
@@ -962,7 +962,7 @@ __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constan
             for (int i = S.start[a] + lane; i < e; i += 32) bump(__ldg(r.adj + i));
           }
           walk_short(r.adj, S.start + S.nlong + 1, S.pre + S.nlong + 1, S.nshort, [&](unsigned w) { bump((int)w); });
-          __syncthreads();
+          block_sync();
           const int slots = 1 << (32 - shift);
           for (int i = tid; i < slots; i += kRT) {
             const unsigned k = keys[i];
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constan
               list_segments(S, nb, st, len);
               here |= S.nlong | S.nshort;
               closed += count_chunk<ORD>(r.adj16, S, lo, lbits, (unsigned)o_max);
-              __syncthreads();
+              block_sync();
 #pragma unroll
               for (int k = 0; k < 4; k++) {
                 const int t = slot_of(k);
@@ -1063,7 +1063,7 @@ __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constan
         }
       }
       owner_end(v);
-      __syncthreads();
+      block_sync();
     }
   }
   if (ORD) {
@@ -1184,13 +1184,6 @@ double exact_bound_log2(const DevGraph& G, const WedgeParams& p) {
   return std::log2((double)std::max(2LL, G.m)) + std::log2(d) + lb(p.f_v) + lb(p.f_vw) + lb(p.f_w) + 2.0;
 }
 
-// Whether no binomial of the pattern over the graph's degrees wraps in u64
-// before its division: C(d, k) k <= d^k / (k-1)! < 2^64.
-bool binomials_exact(const DevGraph& G, const WedgeParams& p) {
-  const int k = std::max(p.f_v, std::max(p.f_vw, p.f_w));
-  return k <= 2 || k * std::log2((double)std::max(2, G.maxdeg)) - std::lgamma((double)k) / std::log(2.0) < 63.0;
-}
-
 PairForm pair_form(const WedgeParams& p, bool exact) {
   const int lo = std::min(p.f_v, p.f_w), k = std::max(p.f_v, p.f_w), s = p.f_vw;
   PairForm f{kGeneral, s, 0, 0, 1};
@@ -1270,7 +1263,7 @@ int enqueue_rank_a(DevGraph& G, const GView& gv, const WedgeParams* pats, u64* c
     rs.w = p;
     rs.lim = p.lim;
     rs.slot[0] = slots[i];
-    const bool fits = std::is_same<A, u128>::value || binomials_exact(G, p);
+    const bool fits = std::is_same<A, u128>::value || binomials_fit(G.maxdeg, std::max(p.f_v, std::max(p.f_vw, p.f_w)));
     rs.form = pair_form(p, fits);
     rs.roles = !fits;  // the sum does not depend on which end is which unless a binomial wraps
     st = launch_rank_set<false, A>(r, rs, G, s, launches, work);
@@ -1280,6 +1273,10 @@ int enqueue_rank_a(DevGraph& G, const GView& gv, const WedgeParams* pats, u64* c
 }
 
 }  // namespace
+
+bool binomials_fit(int maxdeg, int k) {
+  return k <= 2 || k * std::log2((double)std::max(2, maxdeg)) - std::lgamma((double)k) / std::log(2.0) < 63.0;
+}
 
 int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) {
   if (G.radj) return FSGC_OK;

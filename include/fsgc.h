@@ -146,9 +146,8 @@ int fsgc_ctx_set_exact_placements(fsgc_ctx* ctx, int on);
 typedef struct fsgc_tuning {
   int32_t wedge_small_max_degree; /* wedge pairs: endpoints up to this degree (16..2048) count in the
                                      shared-memory kernel, higher ones in the hub kernel */
-  int32_t triangle_walk_ratio;    /* triangle bitmaps: a row walks N(b) against the staged N(a) when
-                                     deg b <= ratio * deg a, else searches N(b) (0: always search) */
-  int32_t triangle_stage_max;     /* longest N(a) staged in shared memory by bulk copy (0..8192, x32) */
+  int32_t triangle_walk_ratio;    /* range-checked and kept; no kernel reads it (0..2^20) */
+  int32_t triangle_stage_max;     /* range-checked and kept; no kernel reads it (0..8192, x32) */
   int32_t general_lane_venn_max;  /* general core: a lane builds its own Venn row up to this many
                                      list entries, longer rows are built by the whole warp */
   int32_t general_blocks_per_sm;  /* general core: resident blocks of 4 warps per SM (1..16) */
