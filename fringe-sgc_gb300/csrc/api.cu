@@ -109,6 +109,7 @@ void free_graph(DevGraph* g) {
   cudaFree(g->ctab_rows);
   cudaFree(g->ctab_pos);
   cudaFree(g->wide);
+  cudaFree(g->bits);
   cudaFree(g->roff);
   cudaFree(g->radj);
   cudaFree(g->rdeg);

@@ -1164,6 +1164,261 @@ __global__ void __launch_bounds__(kGenWarps * 32) general_core_kernel(GView g, c
   block_sum_to(acc, slot);
 }
 
+// ---- general core on a bit matrix (graphs of at most kBitsMaxN vertices)
+//
+// Row v of the matrix is N(v), one bit per vertex.  A candidate is then checked
+// with one bit per core vertex it must (not) touch, where the lists need a
+// binary search each, and the number of vertices adjacent to a set of anchors is
+// a popcount of their rows' AND.  The rows of the anchors before the last core
+// vertex are ANDed once per partial match (without the core vertices), so a
+// match costs one pass over its own row per set that its formula needs:
+//   few     at most three fringes, one per anchor set: the sets and their
+//           unions, F1 F2 - F12 and its three-set counterpart;
+//   others  all sets of anchors (at most four), turned into exclusive regions
+//           for the placement walk.
+// Bound by instructions (popcounts, the walk).  RMAT n = 512, 14,000 entries: a
+// five-vertex core with a chord fringe 45 -> 0.5 ms, a 4-path with three
+// fringes 57 -> 0.5 ms; n = 1,500: 45 -> 0.95 ms.  The matrix stays under 2 MiB.
+constexpr int kBitsMaxN = 4096;
+constexpr int kBitsMaxAnchors = 4;  // for the placement walk
+constexpr int kBitsMaxSets = 15;
+
+struct BitSets {
+  int few;                       // fringes counted by inclusion-exclusion (0: placement walk)
+  int twice;                     // few: the reference's walk starts with its all-anchor step and repeats it
+  int nsets;                     // anchor sets whose common neighbours are counted
+  uint8_t set[kBitsMaxSets];     // as core bitmaps
+  int8_t term[7];                // few: index of F1, F2, F12, F3, F13, F23, F123
+  int parts;                     // ways a list entry's third vertices are split over tasks
+  int words;                     // matrix words per row (a multiple of 4)
+};
+
+struct BitWarp {
+  int stack[6];
+  int before[kBitsMaxSets];  // common neighbours of a set's earlier anchors
+  int venn[32][65];
+};
+
+template <int L, int D, class A>
+__device__ A bits_level(const GView& g, const GenParams& p, const BitSets& bs, const unsigned* __restrict__ mat, BitWarp& w,
+                        unsigned* rows, int part) {
+  const int lane = threadIdx.x & 31;
+  const int words = bs.words;
+  const int list = p.list[L];
+  const int src = w.stack[__ffs(list) - 1];
+  const long long sb = g.off[src];
+  const int sd = (int)(g.off[src + 1] - sb);
+  const bool last = (L + 1 == p.k - 1);
+  const int xbit = 1 << (L + 1);
+  A acc = A(0);
+  if (last) {
+    // per set: the AND of its earlier anchors' rows without the core vertices
+    for (int q = 0; q < bs.nsets; q++) {
+      const int early = bs.set[q] & ~xbit;
+      int c = 0;
+      if (early) {
+        for (int i = lane; i < words; i += 32) {
+          unsigned x = 0xffffffffu;
+          for (int a = 0; a <= L; a++) {
+            const int va = w.stack[a];
+            if (early >> a & 1) x &= __ldg(mat + (size_t)va * words + i);
+            if (va >> 5 == i) x &= ~(1u << (va & 31));
+          }
+          rows[q * words + i] = x;
+          c += __popc(x);
+        }
+      }
+      c = __reduce_add_sync(0xffffffffu, c);
+      if (lane == 0) w.before[q] = c;
+    }
+    __syncwarp();
+  }
+  for (int t0 = 0; t0 < sd; t0 += 32) {
+    const int t = t0 + lane;
+    bool ok = false;
+    int x = 0;
+    if (t < sd && (L > 1 || t % bs.parts == part)) {
+      x = __ldg(g.adj + sb + t);
+      ok = g.deg[x] >= p.destdeg[L];
+      for (int q = 0; q <= L && ok; q++) {
+        const int vq = w.stack[q];
+        ok = (list >> q & 1) ? (__ldg(mat + (size_t)vq * words + (x >> 5)) >> (x & 31)) & 1u : vq != x;
+      }
+    }
+    if (last) {
+      if (ok) {
+        const uint4* mx = reinterpret_cast<const uint4*>(mat + (size_t)x * words);
+        int* row = w.venn[lane];
+        for (int q = 0; q < bs.nsets; q++) {
+          const int set = bs.set[q], early = set & ~xbit;
+          int c;
+          if (!(set & xbit)) {
+            c = w.before[q] - (int)((rows[q * words + (x >> 5)] >> (x & 31)) & 1u);
+          } else if (early == 0) {
+            c = g.deg[x];
+            for (int a = 0; a <= L; a++) {
+              const int va = w.stack[a];
+              c -= (int)((__ldg(mat + (size_t)x * words + (va >> 5)) >> (va & 31)) & 1u);
+            }
+          } else {
+            const uint4* r4 = reinterpret_cast<const uint4*>(rows + q * words);
+            c = 0;
+            for (int i = 0; i < words / 4; i++) {
+              const uint4 a = __ldg(mx + i), b = r4[i];
+              c += (__popc(a.x & b.x) + __popc(a.y & b.y)) + (__popc(a.z & b.z) + __popc(a.w & b.w));
+            }
+          }
+          row[set] = c;
+        }
+        A f;
+        if (bs.few > 0) {
+          // below 2^36, and never negative: exact in any arithmetic
+          auto at = [&](int i) { return (u64)row[bs.set[bs.term[i]]]; };
+          u64 few = at(0);
+          if (bs.few == 2) few = at(0) * at(1) - at(2);
+          if (bs.few == 3) few = at(0) * at(1) * at(3) - at(0) * at(5) - at(1) * at(4) - at(3) * at(2) + 2 * at(6);
+          f = A(bs.twice ? 2 * few : few);
+        } else {
+          // common neighbours of every set -> exclusive regions
+          row[0] = 0;
+          for (int a = 0; a < p.k; a++) {
+            if (!(p.anchors >> a & 1)) continue;
+            for (int q = 0; q < bs.nsets; q++) {
+              const int set = bs.set[q];
+              if (!(set >> a & 1)) row[set] -= row[set | 1 << a];
+            }
+          }
+          f = placement_of<D, A>(p, row);
+        }
+        credit(g, acc, f, w.stack[0]);
+      }
+      __syncwarp();
+    } else {
+      unsigned bal = __ballot_sync(0xffffffffu, ok);
+      while (bal) {
+        const int who = __ffs(bal) - 1;
+        bal &= bal - 1;
+        const int xx = __shfl_sync(0xffffffffu, x, who);
+        if (lane == 0) w.stack[L + 1] = xx;
+        __syncwarp();
+        if constexpr (L < 4) acc += bits_level<L + 1, D, A>(g, p, bs, mat, w, rows, part);
+        __syncwarp();
+      }
+    }
+  }
+  return acc;
+}
+
+// One warp per (list entry, part) task, from a queue.
+template <int D, class A>
+__global__ void __launch_bounds__(kGenWarps * 32) general_bits_kernel(GView g, const __grid_constant__ GenParams p,
+                                                                       const __grid_constant__ BitSets bs,
+                                                                       const unsigned* __restrict__ mat,
+                                                                       unsigned long long* __restrict__ queue,
+                                                                       u64* __restrict__ slot) {
+  extern __shared__ __align__(16) unsigned s_rows[];
+  __shared__ BitWarp sw[kGenWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  BitWarp& w = sw[warp];
+  unsigned* rows = s_rows + (size_t)warp * bs.nsets * bs.words;
+  A acc = A(0);
+  const unsigned long long tasks = (unsigned long long)g.m * (unsigned)bs.parts;
+  for (;;) {
+    unsigned long long task = 0;
+    if (lane == 0) task = atomicAdd(queue, 1ULL);
+    task = __shfl_sync(0xffffffffu, task, 0);
+    if (task >= tasks) break;
+    const long long j = (long long)(task / (unsigned)bs.parts);
+    int lo = 0, hi = g.n;  // owner: the last vertex with off[u] <= j
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (g.off[mid] <= j) lo = mid;
+      else hi = mid;
+    }
+    const int v = __ldg(g.adj + j);
+    if (g.deg[lo] < p.startdeg || g.deg[v] < p.destdeg[0]) continue;  // init_wl_general
+    if (lane == 0) {
+      w.stack[0] = lo;
+      w.stack[1] = v;
+    }
+    __syncwarp();
+    acc += bits_level<1, D, A>(g, p, bs, mat, w, rows, (int)(task % (unsigned)bs.parts));
+    __syncwarp();
+  }
+  block_sum_to(acc, slot);
+}
+
+__global__ void bit_matrix_kernel(GView g, int words, unsigned* __restrict__ mat) {
+  const int lane = threadIdx.x & 31;
+  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int v = wid; v < g.n; v += nw) {
+    const long long b = g.off[v];
+    for (int t = lane; t < g.deg[v]; t += 32) {
+      const int x = __ldg(g.adj + b + t);
+      if ((unsigned)x < (unsigned)g.n) atomicOr(mat + (size_t)v * words + (x >> 5), 1u << (x & 31));
+    }
+  }
+}
+
+int bit_matrix_words(int n) { return ((n + 31) / 32 + 3) & ~3; }
+
+// The adjacency bit matrix of a small graph, once per graph (at most 2 MiB).
+int ensure_bit_matrix(DevGraph& G, cudaStream_t s, uint64_t* launches) {
+  if (G.bits) return FSGC_OK;
+  const size_t bytes = sizeof(unsigned) * (size_t)G.n * bit_matrix_words(G.n);
+  if (cudaMallocAsync((void**)&G.bits, bytes, s) != cudaSuccess) {
+    cudaGetLastError();
+    G.bits = nullptr;
+    return FSGC_ENOMEM;
+  }
+  cudaMemsetAsync(G.bits, 0, bytes, s);
+  bit_matrix_kernel<<<std::max(1, std::min(G.n / 8 + 1, sm_count() * 8)), 256, 0, s>>>(G.view(), bit_matrix_words(G.n), G.bits);
+  *launches += 1;
+  G.bytes += bytes;
+  return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
+}
+
+// The sets a pattern needs counted, or false when it takes the list kernel.  With
+// one fringe per set the reference's walk is exact but for one case: when its
+// first step is the all-anchor one and other sets follow, that step's saved
+// alternative starts at 1 instead of 0 and the walk below it runs twice.
+bool bit_sets_for(const GenParams& p, bool exact, int n, BitSets& bs) {
+  if (n > kBitsMaxN) return false;
+  memset(&bs, 0, sizeof(bs));
+  bs.words = bit_matrix_words(n);
+  bool ones = p.nsets <= 3;
+  for (int i = 0; i < p.nsets; i++) ones = ones && p.fcnt[i] == 1;
+  auto need = [&](int set) {
+    for (int q = 0; q < bs.nsets; q++)
+      if (bs.set[q] == set) return q;
+    bs.set[bs.nsets] = (uint8_t)set;
+    return bs.nsets++;
+  };
+  if (ones) {
+    bs.few = p.nsets;
+    bs.twice = !exact && p.nsets > 1 && p.slot_top[0];
+    const int a = p.anch[0], b = p.nsets > 1 ? p.anch[1] : 0, c = p.nsets > 2 ? p.anch[2] : 0;
+    const int sets[7] = {a, b, a | b, c, a | c, b | c, a | b | c};
+    const bool used[7] = {true, p.nsets > 1, p.nsets > 1, p.nsets > 2, p.nsets > 2, p.nsets > 2, p.nsets > 2};
+    for (int i = 0; i < 7; i++)
+      if (used[i]) bs.term[i] = (int8_t)need(sets[i]);
+    return true;
+  }
+  if (__builtin_popcount(p.anchors) > kBitsMaxAnchors) return false;
+  for (int set = 1; set < 64; set++)
+    if ((set & ~p.anchors) == 0) need(set);
+  return true;
+}
+
+template <int D, class A>
+int launch_bits(const GView& gv, const GenParams& gp, BitSets bs, const unsigned* mat, unsigned long long* queue, u64* slot,
+                int blocks, cudaStream_t s) {
+  const size_t smem = sizeof(unsigned) * (size_t)kGenWarps * bs.nsets * bs.words;
+  cudaFuncSetAttribute(general_bits_kernel<D, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  general_bits_kernel<D, A><<<blocks, kGenWarps * 32, smem, s>>>(gv, gp, bs, mat, queue, slot);
+  return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
+}
+
 // ------------------------------------------------------------- host helpers
 void rotations3(const int f[8], bool wedge, Rot3& r) {
   auto rot = [](const int* q, int* o) {
@@ -1265,6 +1520,7 @@ struct Needs {
   bool chunk_table = false;  // wedge core with a fringe-free centre
   bool vertex_triangles = false;
   bool entry_supports = false;  // general wedge core
+  bool bit_matrix = false;      // general core of a small graph
   size_t scratch = 0;        // arena bytes (hub cursors, triangle bitmaps)
 };
 
@@ -1278,7 +1534,10 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
     if (f_uv == 1 && (f_u == 0 || f_v == 0)) nd.vertex_triangles = !(f_u == 0 && f_v == 0) || G.ngraphs > 0;
     return nd;
   }
-  if (mo.nodes > 3) return nd;
+  if (mo.nodes > 3) {
+    nd.bit_matrix = G.n <= kBitsMaxN;
+    return nd;
+  }
   int f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (int i = 0; i < mo.anchorsets; i++) f[mo.anch[i] & 7] = mo.fcnt[i];
   if (__builtin_popcount(mo.list[1]) == 1) {
@@ -1340,6 +1599,10 @@ int prepare_for_count(const fsgc_matching_order& mo, DevGraph& G, cudaStream_t s
     st = ensure_entry_supports(G, s, launches);
     if (st != FSGC_OK) return st;
   }
+  if (nd.bit_matrix) {
+    st = ensure_bit_matrix(G, s, launches);
+    if (st != FSGC_OK) return st;
+  }
   return cudaStreamSynchronize(s) == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
 
@@ -1352,6 +1615,7 @@ int prepare_all(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) 
   }
   if (st == FSGC_OK) st = ensure_vertex_triangles(G, s, launches);
   if (st == FSGC_OK && G.ngraphs == 0) st = ensure_entry_supports(G, s, launches);
+  if (st == FSGC_OK && G.n <= kBitsMaxN) st = ensure_bit_matrix(G, s, launches);
   if (st != FSGC_OK) return st;
   return cudaStreamSynchronize(s) == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
@@ -1562,6 +1826,26 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
   const int blocks = sm_count() * std::min(16, std::max(1, work.tune.general_blocks_per_sm));
   // one edge per grab until there are many more edges than warps
   gp->grab = (int)std::max(1LL, std::min(32LL, G.m / ((long long)blocks * kGenWarps * 64)));
+  BitSets bs;
+  if (bit_sets_for(*gp, gp->exact || !std::is_same<A, u64>::value, G.n, bs)) {
+    st = ensure_bit_matrix(G, s, launches);
+    if (st == FSGC_OK) {
+      // enough tasks for the warps to end together
+      bs.parts = 1;
+      while (bs.parts < 32 && G.m * bs.parts < (long long)blocks * kGenWarps * 32) bs.parts *= 2;
+      if (ns <= 32) st = launch_bits<32, A>(gv, *gp, bs, G.bits, queue, job.d_slot, blocks, s);
+      else if (ns <= 64) st = launch_bits<64, A>(gv, *gp, bs, G.bits, queue, job.d_slot, blocks, s);
+      else st = launch_bits<128, A>(gv, *gp, bs, G.bits, queue, job.d_slot, blocks, s);
+      *launches += 1;
+      delete gp;
+      return st;
+    }
+    if (st != FSGC_ENOMEM) {
+      delete gp;
+      return st;
+    }
+    st = FSGC_OK;  // no room for the matrix: the lists
+  }
   // the placement walk's state is sized by the step count
   if (ns <= 32) general_core_kernel<32, A><<<blocks, kGenWarps * 32, 0, s>>>(gv, *gp, queue, job.d_slot);
   else if (ns <= 64) general_core_kernel<64, A><<<blocks, kGenWarps * 32, 0, s>>>(gv, *gp, queue, job.d_slot);
