@@ -7,7 +7,8 @@
 // changes is how the matches and their Venn sizes are found:
 //   vertex core   one pass over the degrees;
 //   edge core     one pass over oriented edges, common-neighbour counts taken
-//                 from the loader's per-edge triangle supports;
+//                 from the loader's per-edge triangle supports, binomials in
+//                 chains;
 //   triangle core bitmap rows per lowest vertex (triangle.cu); here only for
 //                 out-degrees beyond its tables;
 //   wedge core    (centre without fringes) aggregated per endpoint pair: the
@@ -54,6 +55,86 @@ struct EdgeParams {
   int f_u, f_uv, f_v, lim1, lim2;
 };
 
+
+// C(n, 0..K) as nck_ref(n, k) gives them, in one chain: its r after step i is
+// C(n, i) with the wrapping of every step, whatever k it is on the way to, and
+// below n = 2 k, where it goes to n - k instead, nothing wraps.  n >= 0.
+template <int K>
+__device__ __forceinline__ void binomial_chain(int n, u64* c) {
+  c[0] = 1;
+  if constexpr (K >= 1) c[1] = (u64)n;
+  if constexpr (K >= 2) c[2] = ((u64)n * (u64)(n - 1)) >> 1;
+#pragma unroll
+  for (int i = 3; i <= K; i++) c[i] = c[i - 1] * (u64)(n + 1 - i) / (u64)i;
+}
+
+// C(n - j, F) as nck_ref gives them, j = 0..J, n >= 0; where j > n any value.
+// Up to n = nfit nothing below k = F wraps: C(n - j, k) then follows from
+// C(n - j + 1, k) by a subtraction, and only the step to F is done as nck_ref
+// does it.
+template <int F, int J>
+__device__ __forceinline__ void binomial_column(int n, int nfit, u64* t) {
+  if constexpr (F <= 2) {
+#pragma unroll
+    for (int j = 0; j <= J; j++)
+      t[j] = F == 0 ? 1ULL : F == 1 ? (u64)(n - j) : ((u64)(n - j) * (u64)(n - j - 1)) >> 1;
+  } else if (n <= nfit) {
+    u64 c[F];
+    binomial_chain<F - 1>(n, c);
+#pragma unroll
+    for (int j = 0; j <= J; j++) {
+      if (j > 0) {
+#pragma unroll
+        for (int k = 1; k < F; k++) c[k] -= c[k - 1];  // ascending: c[k - 1] is the new row's
+      }
+      t[j] = c[F - 1] * (u64)(n - j + 1 - F) / (u64)F;
+    }
+  } else {
+    for (int j = 0; j <= J; j++) t[j] = nck(n - j, F);
+  }
+}
+
+// edge_formula for few fringes, each binomial once: the formula's pool
+// a_uv + c_v - j is deg v - 1 - f_uv - j.  Bound by instructions (350 a warp,
+// 73 % of the SMs' issue rate; the 12 bytes an edge would take 28 us): five
+// fringes on each end, RMAT n = 2^20, 15.7 M edges, 1.42 -> 0.29 ms against the
+// loop of nck calls, which lanes leave at different steps.  More than six
+// fringes on an end keep the loop: their columns' state would spill.
+template <int FU, int FV>
+__device__ __forceinline__ u64 edge_formula_chains(int du, int dv, int c_uv, int f_uv, int nfit) {
+  const int a_uv = c_uv - f_uv;
+  if (a_uv < 0) return 0;
+  u64 ku[FU + 1], b[FU + 1], t[FU + 1];
+  binomial_chain<FU>(a_uv, b);  // 0 beyond a_uv
+  binomial_chain<FU>(du - 1 - c_uv, ku);
+  binomial_column<FV, FU>(dv - 1 - f_uv, nfit, t);
+  u64 acc = 0;
+#pragma unroll
+  for (int j = 0; j <= FU; j++) acc += ku[FU - j] * t[j] * b[j];
+  if constexpr (FU != FV) {
+    binomial_chain<FU>(dv - 1 - c_uv, ku);
+    binomial_column<FV, FU>(du - 1 - f_uv, nfit, t);
+#pragma unroll
+    for (int j = 0; j <= FU; j++) acc += ku[FU - j] * t[j] * b[j];
+  }
+  return acc * nck(c_uv, f_uv);
+}
+
+constexpr int kEdgeChainMax = 6;  // fringes of one endpoint
+
+template <int FU, int FV>
+__global__ void __launch_bounds__(kTPB) edge_chain_kernel(GView g, EdgeParams p, int nfit, u64* __restrict__ slot) {
+  const long long me = g.m / 2;
+  u64 acc = 0;
+  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < me; j += (long long)gridDim.x * blockDim.x) {
+    const int a = g.osrc[j], b = g.oadj[j];
+    const int u = max(a, b), v = min(a, b);  // the reference orients by id, v < u
+    const int du = g.deg[u], dv = g.deg[v];
+    if (!(du > p.lim1 && dv > p.lim1 && du + dv > p.lim2)) continue;  // init_wl_edge pruning
+    credit(g, acc, edge_formula_chains<FU, FV>(du, dv, (int)g.osup[j], p.f_uv, nfit), a);
+  }
+  block_sum_to(acc, slot);
+}
 
 template <class A>
 __global__ void edge_kernel(GView g, EdgeParams p, u64* __restrict__ slot) {
@@ -1455,6 +1536,21 @@ int grid_for(long long work, int tpb, int per_sm) {
   return (int)std::max(1LL, std::min(want, cap));
 }
 
+// The instantiation of the pattern's fringe counts, f_u <= f_v <= kEdgeChainMax.
+template <int FU, int FV>
+void launch_edge_chains(const GView& gv, const EdgeParams& ep, u64* slot, cudaStream_t s) {
+  if (ep.f_u > FU) {
+    if constexpr (FU < kEdgeChainMax) launch_edge_chains<FU + 1, FU + 1>(gv, ep, slot, s);
+  } else if (ep.f_v > FV) {
+    if constexpr (FV < kEdgeChainMax) launch_edge_chains<FU, FV + 1>(gv, ep, slot, s);
+  } else {
+    int nfit = 0;  // the largest n without wrapping below FV
+    for (int bit = 30; bit >= 0; bit--)
+      if (binomials_fit(nfit | 1 << bit, FV - 1)) nfit |= 1 << bit;
+    edge_chain_kernel<FU, FV><<<grid_for(gv.m / 2, kTPB, 8), kTPB, 0, s>>>(gv, ep, nfit, slot);
+  }
+}
+
 // Builds the wedge core's chunk-boundary table once per graph (vertices of
 // degree >= 512, fewer when the table would pass 512 MiB).
 int ensure_chunk_table(DevGraph& G, cudaStream_t s, uint64_t* launches, u64* d_small) {
@@ -1722,7 +1818,10 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
     }
     EdgeParams ep{f_u, f_uv, f_v, f_u + f_uv, f_u + f_uv + f_v};
     if (me > 0) {
-      edge_kernel<A><<<grid_for(me, TPB, 8), TPB, 0, s>>>(gv, ep, job.d_slot);
+      if (std::is_same<A, u64>::value && f_v <= kEdgeChainMax)
+        launch_edge_chains<0, 0>(gv, ep, job.d_slot, s);
+      else
+        edge_kernel<A><<<grid_for(me, TPB, 8), TPB, 0, s>>>(gv, ep, job.d_slot);
       *launches += 1;
     }
     return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
@@ -1940,6 +2039,19 @@ int enqueue_count_set(std::vector<CountJob*>& jobs, cudaStream_t s, uint64_t* la
     vertex_set_kernel<<<grid_for(G.n, TPB, 8), TPB, 0, s>>>(gv, tailed ? G.vtri2 : nullptr, vs);
     *launches += 1;
   }
+  // few fringes: a kernel each.  A pass for two patterns takes 32 us over 8,000
+  // edges and 127 us over 3.2 M in the fused kernel's nck loops, 27 and 101 us in
+  // two kernels (whole calls).
+  auto fused = edges.begin();
+  for (auto& e : edges) {
+    if (e.second.f_v > kEdgeChainMax || G.m == 0) {
+      *fused++ = e;
+      continue;
+    }
+    launch_edge_chains<0, 0>(gv, e.second, e.first->d_slot, s);
+    *launches += 1;
+  }
+  edges.erase(fused, edges.end());
   for (size_t b = 0; b < edges.size(); b += kPassFuse) {
     EdgeSet es;
     memset(&es, 0, sizeof(es));
