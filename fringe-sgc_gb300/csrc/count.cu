@@ -17,7 +17,8 @@
 //                 evaluated once and multiplied by its number of centres: in
 //                 rank order (wedge_rank.cu), here for graphs that do not take
 //                 that path;
-//                 (centre with fringes) one warp per centre-endpoint edge;
+//                 (centre with fringes) one warp per centre-endpoint edge, on
+//                 the bit matrix of a small graph;
 //   general core  warp-cooperative depth-first matching of 4-6 core vertices,
 //                 a Venn histogram per match and a per-lane placement sum.
 #include <algorithm>
@@ -810,6 +811,7 @@ __global__ void chunk_table_fill_kernel(GView g, const int* __restrict__ rows, i
 struct GWedgeParams {
   int min_u, lim, sum1, sum2, sum3;
   Rot3 rot;
+  u64 packed[6];  // the rotations' counts, a byte each
 };
 
 // Centre with fringes (general_wedge_core, src/fringeCount.cu:1480-1650): one
@@ -1259,7 +1261,9 @@ __global__ void __launch_bounds__(kGenWarps * 32) general_core_kernel(GView g, c
 //           for the placement walk.
 // Bound by instructions (popcounts, the walk).  RMAT n = 512, 14,000 entries: a
 // five-vertex core with a chord fringe 45 -> 0.5 ms, a 4-path with three
-// fringes 57 -> 0.5 ms; n = 1,500: 45 -> 0.95 ms.  The matrix stays under 2 MiB.
+// fringes 57 -> 0.5 ms; n = 1,500: 45 -> 0.95 ms.  Up to 4,096 vertices the matrix
+// stays under 2 MiB and a row within the four words a lane that the wedge core
+// keeps in registers.
 constexpr int kBitsMaxN = 4096;
 constexpr int kBitsMaxAnchors = 4;  // for the placement walk
 constexpr int kBitsMaxSets = 15;
@@ -1444,13 +1448,17 @@ __global__ void bit_matrix_kernel(GView g, int words, unsigned* __restrict__ mat
 int bit_matrix_words(int n) { return ((n + 31) / 32 + 3) & ~3; }
 
 // The adjacency bit matrix of a small graph, once per graph (at most 2 MiB).
+// FSGC_EUNSUPPORTED when the graph is larger or there was no room for it: the
+// caller takes the lists.
 int ensure_bit_matrix(DevGraph& G, cudaStream_t s, uint64_t* launches) {
   if (G.bits) return FSGC_OK;
+  if (G.bits_failed || G.n > kBitsMaxN) return FSGC_EUNSUPPORTED;
   const size_t bytes = sizeof(unsigned) * (size_t)G.n * bit_matrix_words(G.n);
   if (cudaMallocAsync((void**)&G.bits, bytes, s) != cudaSuccess) {
     cudaGetLastError();
     G.bits = nullptr;
-    return FSGC_ENOMEM;
+    G.bits_failed = true;
+    return FSGC_EUNSUPPORTED;
   }
   cudaMemsetAsync(G.bits, 0, bytes, s);
   bit_matrix_kernel<<<std::max(1, std::min(G.n / 8 + 1, sm_count() * 8)), 256, 0, s>>>(G.view(), bit_matrix_words(G.n), G.bits);
@@ -1498,6 +1506,146 @@ int launch_bits(const GView& gv, const GenParams& gp, BitSets bs, const unsigned
   cudaFuncSetAttribute(general_bits_kernel<D, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   general_bits_kernel<D, A><<<blocks, kGenWarps * 32, smem, s>>>(gv, gp, bs, mat, queue, slot);
   return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
+}
+
+// ---- wedge core with a fringed centre on the bit matrix
+//
+// The matches, thresholds and values of wedge_general_kernel, whose time went
+// into walking the shorter of N(v), N(w) with two binary searches per entry for
+// every match.  Here the warp of a list entry (u, v) keeps the rows of v and of
+// N(u) & N(v) in registers, and a match costs its row once, read together, and
+// two popcounts a word; the lanes' matches are then evaluated at one place.
+// Bound by instructions (60 % of the issue rate, 44 % of the warps in flight).
+// One fringe on each of the three, RMAT n = 3,001, 16 entries a vertex: 3.93 ms
+// -> 0.39 ms by fc3_ring in line, 0.25 ms by the products.
+// NW: words of a row per lane.  FORM: 0 fc3; while no binomial wraps, 1 when the
+// fringes on single core vertices are at most one each and there are none on
+// pairs (products), 2 fc3_ring otherwise, out of line: its loops spill.
+__device__ __noinline__ u64 fc3_ring_call(u64 fr, int r, int uv, int uw, int vw, int xu, int xv, int xw) {
+  int f[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) f[i] = (int)(fr >> (8 * i) & 0xff);
+  return fc3_ring(f, r, uv, uw, vw, xu, xv, xw);
+}
+
+// fc3_ring with at most one fringe on each core vertex and none on pairs.
+__device__ __forceinline__ u64 fc3_ones(const int* fr, int r, int uv, int uw, int vw, int xu, int xv, int xw) {
+  const int fuvw = fr[IUVW];
+  if (r < fuvw) return 0;
+  const u64 base = nck(r, fuvw);
+  r -= fuvw;
+  const u64 a = (u64)(unsigned)(r + uv + uw + xu), b = (u64)(unsigned)(r + uv + vw + xv), c = (u64)(unsigned)(r + uw + vw + xw);
+  const u64 ab = (u64)(unsigned)(r + uv), ac = (u64)(unsigned)(r + uw), bc = (u64)(unsigned)(r + vw);
+  u64 x = fr[IU] ? a : 1;
+  if (fr[IV]) x *= b;
+  if (fr[IW]) x *= c;
+  // less the choices that coincide
+  if (fr[IU] & fr[IV]) x -= ab * (fr[IW] ? c : 1);
+  if (fr[IU] & fr[IW]) x -= ac * (fr[IV] ? b : 1);
+  if (fr[IV] & fr[IW]) x -= bc * (fr[IU] ? a : 1);
+  if (fr[IU] & fr[IV] & fr[IW]) x += 2ULL * (u64)(unsigned)r;
+  return base * x;
+}
+
+template <int NW, int FORM, class A>
+__global__ void __launch_bounds__(kTPB) wedge_bits_kernel(GView g, const __grid_constant__ GWedgeParams p, const unsigned* __restrict__ esup,
+                                                           const unsigned* __restrict__ mat, int words,
+                                                           u64* __restrict__ slot) {
+  const int lane = threadIdx.x & 31;
+  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  A acc = A(0);
+  for (long long j = wid; j < g.m; j += nw) {
+    int lo = 0, hi = g.n;  // u = the last vertex with off[u] <= j
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (g.off[mid] <= j) lo = mid;
+      else hi = mid;
+    }
+    const int u = lo, v = __ldg(g.adj + j);
+    const int du = g.deg[u], dv = g.deg[v];
+    if (du < p.sum1 || dv < max(p.sum1, p.sum2 - du)) continue;  // init_wl_wedge
+    const long long ub = g.off[u];
+    const unsigned* row_v = mat + (size_t)v * words;
+    unsigned bv[NW], buv[NW];
+#pragma unroll
+    for (int i = 0; i < NW; i++) {
+      const int word = i * 32 + lane;
+      bv[i] = word < words ? __ldg(row_v + word) : 0;
+      buv[i] = word < words ? bv[i] & __ldg(mat + (size_t)u * words + word) : 0;
+    }
+    const int p12 = (int)__ldg(esup + j);  // |N(u) & N(v)|
+    const bool cond = (du >= p.min_u) && (dv >= p.lim);
+    const int thres1 = max(p.lim, p.sum2 - dv);
+    const int thres2 = max(max(p.sum1, p.sum3 - du - dv), max(p.sum2 - du, p.sum2 - dv));
+    const int ahead = (int)(j - ub);  // w < v: the entries before v's
+    for (int t0 = 0; t0 < ahead; t0 += 32) {
+      const int t = t0 + lane;
+      bool active = false, tri = false;
+      int w = 0, dw = 0, t13 = 0;
+      if (t < ahead) {
+        w = __ldg(g.adj + ub + t);
+        dw = g.deg[w];
+        if (dw >= thres2) {
+          tri = (__ldg(row_v + (w >> 5)) >> (w & 31)) & 1u;
+          active = tri ? (u < w) : (cond && dw >= thres1);
+        }
+        t13 = (int)__ldg(esup + ub + t);
+      }
+      unsigned bal = __ballot_sync(0xffffffffu, active);
+      int both = 0;  // |N(v) & N(w)| and, above 16 bits, |N(u) & N(v) & N(w)|
+      while (bal) {
+        const int who = __ffs(bal) - 1;
+        bal &= bal - 1;
+        const unsigned* row_w = mat + (size_t)__shfl_sync(0xffffffffu, w, who) * words;
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < NW; i++) {
+          const int word = i * 32 + lane;
+          const unsigned x = word < words ? __ldg(row_w + word) : 0;
+          c += __popc(x & bv[i]) + (__popc(x & buv[i]) << 16);
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == who) both = c;
+      }
+      if (!__any_sync(0xffffffffu, active)) continue;
+      // common3_wedge (src/fringeCount.cu:1480-1510) + corrections
+      const int c123 = both >> 16, c12 = p12 - c123, c13 = t13 - c123, c23 = (both & 0xffff) - c123;
+      int xu = du - (p12 + c13), xv = dv - (p12 + c23), xw = dw - (c13 + c23 + c123);
+      int uv = c12, uw = c13, vw = c23;
+      if (tri) {
+        uv--; uw--; vw--;
+      } else {
+        xu -= 2; vw--;
+      }
+      A sum = A(0);
+#pragma unroll 1
+      for (int r = 0; r < p.rot.count; r++) {
+        if (!active || !(tri || r == 0 || r == 3)) continue;
+        if constexpr (FORM == 1) {
+          sum += fc3_ones(p.rot.fr[r], c123, uv, uw, vw, xu, xv, xw);
+        } else if constexpr (FORM == 2) {
+          sum += fc3_ring_call(p.packed[r], c123, uv, uw, vw, xu, xv, xw);
+        } else {
+          const int venn[8] = {0, xu, xv, uv, xw, uw, vw, c123};
+          sum += fc3<A>(p.rot.fr[r], venn);
+        }
+      }
+      if (active) credit(g, acc, sum, u);
+    }
+  }
+  block_sum_to(acc, slot);
+}
+
+template <int NW, class A>
+void launch_wedge_bits(const GView& gv, const GWedgeParams& gp, const unsigned* esup, const unsigned* mat, int words,
+                       int form, u64* slot, int blocks, cudaStream_t s) {
+  if constexpr (std::is_same<A, u64>::value) {
+    if (form == 1) wedge_bits_kernel<NW, 1, A><<<blocks, kTPB, 0, s>>>(gv, gp, esup, mat, words, slot);
+    if (form == 2) wedge_bits_kernel<NW, 2, A><<<blocks, kTPB, 0, s>>>(gv, gp, esup, mat, words, slot);
+    if (form != 0) return;
+  }
+  wedge_bits_kernel<NW, 0, A><<<blocks, kTPB, 0, s>>>(gv, gp, esup, mat, words, slot);
 }
 
 // ------------------------------------------------------------- host helpers
@@ -1616,7 +1764,7 @@ struct Needs {
   bool chunk_table = false;  // wedge core with a fringe-free centre
   bool vertex_triangles = false;
   bool entry_supports = false;  // general wedge core
-  bool bit_matrix = false;      // general core of a small graph
+  bool bit_matrix = false;      // general cores and that one, on a small graph
   size_t scratch = 0;        // arena bytes (hub cursors, triangle bitmaps)
 };
 
@@ -1631,7 +1779,7 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
     return nd;
   }
   if (mo.nodes > 3) {
-    nd.bit_matrix = G.n <= kBitsMaxN;
+    nd.bit_matrix = true;
     return nd;
   }
   int f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -1649,6 +1797,7 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
       }
     } else {
       nd.entry_supports = true;
+      nd.bit_matrix = true;
     }
     return nd;
   }
@@ -1697,7 +1846,7 @@ int prepare_for_count(const fsgc_matching_order& mo, DevGraph& G, cudaStream_t s
   }
   if (nd.bit_matrix) {
     st = ensure_bit_matrix(G, s, launches);
-    if (st != FSGC_OK) return st;
+    if (st != FSGC_OK && st != FSGC_EUNSUPPORTED) return st;
   }
   return cudaStreamSynchronize(s) == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
@@ -1711,7 +1860,10 @@ int prepare_all(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) 
   }
   if (st == FSGC_OK) st = ensure_vertex_triangles(G, s, launches);
   if (st == FSGC_OK && G.ngraphs == 0) st = ensure_entry_supports(G, s, launches);
-  if (st == FSGC_OK && G.n <= kBitsMaxN) st = ensure_bit_matrix(G, s, launches);
+  if (st == FSGC_OK) {
+    st = ensure_bit_matrix(G, s, launches);
+    if (st == FSGC_EUNSUPPORTED) st = FSGC_OK;
+  }
   if (st != FSGC_OK) return st;
   return cudaStreamSynchronize(s) == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
@@ -1857,9 +2009,27 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
     GWedgeParams gp;
     gp.min_u = min_u; gp.lim = lim; gp.sum1 = sum1; gp.sum2 = sum2; gp.sum3 = sum3;
     rotations3(f, true, gp.rot);
+    for (int r = 0; r < gp.rot.count; r++) {
+      gp.packed[r] = 0;
+      for (int i = 1; i < 8; i++) gp.packed[r] |= (u64)gp.rot.fr[r][i] << (8 * i);
+    }
     st = ensure_entry_supports(G, s, launches);
     if (st != FSGC_OK) return st;
-    wedge_general_kernel<A><<<grid_for(G.m * 32, TPB, 8), TPB, 0, s>>>(gv, gp, G.esup, job.d_slot);
+    const int blocks = grid_for(G.m * 32, TPB, 8);
+    st = ensure_bit_matrix(G, s, launches);
+    if (st != FSGC_OK && st != FSGC_EUNSUPPORTED) return st;
+    if (st == FSGC_OK) {
+      int k = 0;
+      for (int i = 0; i < 8; i++) k = std::max(k, f[i]);
+      const bool ones = std::max(f[IU], std::max(f[IV], f[IW])) <= 1 && f[IUV] + f[IUW] + f[IVW] == 0;
+      const int ring = !binomials_fit(G.maxdeg, k) ? 0 : ones ? 1 : 2;
+      const int words = bit_matrix_words(G.n);
+      if (words <= 32) launch_wedge_bits<1, A>(gv, gp, G.esup, G.bits, words, ring, job.d_slot, blocks, s);
+      else if (words <= 64) launch_wedge_bits<2, A>(gv, gp, G.esup, G.bits, words, ring, job.d_slot, blocks, s);
+      else launch_wedge_bits<4, A>(gv, gp, G.esup, G.bits, words, ring, job.d_slot, blocks, s);
+    } else {
+      wedge_general_kernel<A><<<blocks, TPB, 0, s>>>(gv, gp, G.esup, job.d_slot);
+    }
     *launches += 1;
     return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
   }
@@ -1939,7 +2109,7 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
       delete gp;
       return st;
     }
-    if (st != FSGC_ENOMEM) {
+    if (st != FSGC_EUNSUPPORTED) {
       delete gp;
       return st;
     }

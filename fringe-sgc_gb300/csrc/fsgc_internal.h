@@ -69,7 +69,8 @@ struct DevGraph {
   int* rtab = nullptr;  // boundary table of the first rrows lists, rK columns
   int rrows = 0, rK = 0;
   bool rank_failed = false;  // no room for the copy: not tried again
-  unsigned* bits = nullptr;  // lazily: adjacency bit matrix of a small graph (general core)
+  unsigned* bits = nullptr;  // lazily: adjacency bit matrix of a small graph (general cores)
+  bool bits_failed = false;  // no room for it: not tried again
   // the reference's degree-relabel gate for the triangle core
   // (src/fringeCount.cu:1237, 1342-1344): vertex roles follow (deg, id) order
   // when it fires, vertex ids otherwise
