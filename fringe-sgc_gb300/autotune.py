@@ -6,10 +6,10 @@ per context, and this module picks them per graph by timing:
 
   wedge_small_max_degree  endpoint degree up to which the wedge-pair counting
                           runs in the shared-memory counter kernel (higher
-                          degrees go to the hub kernel)
-  triangle_walk_ratio     triangle bitmaps: walk N(b) against the staged N(a)
-                          when deg b <= ratio * deg a, else binary-search N(b)
-  triangle_stage_max      longest N(a) staged in shared memory by bulk copy
+                          degrees go to the hub kernel) on graphs that do not
+                          take the rank-order path
+  triangle_walk_ratio,    kept for saved settings; no kernel reads them, so
+  triangle_stage_max      the default wins unless timing noise says otherwise
   general_lane_venn_max   general cores: Venn rows up to this many list
                           entries are built by one lane, longer ones by a warp
   general_blocks_per_sm   general cores: the task granularity of the grid
