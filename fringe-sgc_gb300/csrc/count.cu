@@ -529,7 +529,7 @@ __device__ void block_scan_inplace(int* x, int n, WedgeSmem<BIG>& S) {
       if (lane >= o) inc += y;
     }
     if (lane == 31) S.warp_tmp[warp] = inc;
-    __syncthreads();
+    block_sync();
     if (warp == 0) {
       const int wv = (lane < nwarp) ? S.warp_tmp[lane] : 0;
       int wi = wv;
@@ -540,12 +540,12 @@ __device__ void block_scan_inplace(int* x, int n, WedgeSmem<BIG>& S) {
       if (lane < nwarp) S.warp_tmp[lane] = wi - wv;
       if (lane == 31) S.warp_tmp[32] = wi;
     }
-    __syncthreads();
+    block_sync();
     const int ex = carry + S.warp_tmp[warp] + inc - sum;
     if (i0 < n) x[i0] = ex;
     if (i1 < n) x[i1] = ex + x0;
     carry += S.warp_tmp[32];
-    __syncthreads();
+    block_sync();
   }
   if (tid == 0) x[n] = carry;
 }
@@ -598,12 +598,12 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
       S.v = atomicAdd(queue, 1);
       S.lo = 0;
     }
-    __syncthreads();
+    block_sync();
     const int v = S.v;
     if (v >= g.n) break;
     const int dv = g.deg[v];
     if (dv < ws.lim || (BIG ? dv <= ws.small_max : dv > ws.small_max)) {
-      __syncthreads();
+      block_sync();
       continue;
     }
     // counter layout: `bits` per counter, 2^lper counters per word, CH ids per chunk
@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
       lim[t] = g.off[u + 1];
     }
     int cv = 0;  // cursor into N(v) for the adjacency marks
-    __syncthreads();
+    block_sync();
     while (S.lo < v) {
       const int lo = S.lo;  // a multiple of CH
       const int hi = min(lo + CH, v);
@@ -642,9 +642,9 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
         const int o = __ldg(Nv + i) - lo;
         atomicOr(&S.adjbits[o >> 5], 1u << (o & 31));
       }
-      __syncthreads();
+      block_sync();
       block_scan_inplace<BIG>(pre, dv, S);
-      __syncthreads();
+      block_sync();
       // count: warp-contiguous ranges of the chunk's elements
       {
         const int L = pre[dv];
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
           }
         }
       }
-      __syncthreads();
+      block_sync();
       // evaluate: the chunk's touched counter words are numbered by a prefix
       // over the touched-bitmap words; a warp takes 32 words at a time, one
       // per lane, prefix-sums their non-zero counters, writes
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
           if (lane >= o) inc += y;
         }
         if (lane == 31) S.warp_tmp[warp] = inc;
-        __syncthreads();
+        block_sync();
         if (warp == 0) {
           const int wv = (lane < nwarp) ? S.warp_tmp[lane] : 0;
           int wi = wv;
@@ -698,11 +698,11 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
           if (lane < nwarp) S.warp_tmp[lane] = wi - wv;
           if (lane == 31) S.warp_tmp[32] = wi;
         }
-        __syncthreads();
+        block_sync();
         S.tpre[tid] = S.warp_tmp[warp] + inc - c0;
         const int T = S.warp_tmp[32];
         if (tid == 0) S.grab = 0;
-        __syncthreads();
+        block_sync();
         const int lbits = BIG ? 5 : (lper == 1 ? 4 : (lper == 2 ? 3 : 2));  // log2(bits)
         const unsigned cmask = BIG ? 0xffffffffu : ((1u << bits) - 1);
         using PT = WedgePair<BIG>;
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
       }
       nxt = __reduce_min_sync(0xffffffffu, nxt);
       if (tid == 0) S.lo = v;
-      __syncthreads();  // touched, adjbits, pre and S.lo are free again
+      block_sync();  // touched, adjbits, pre and S.lo are free again
       for (int i = tid; i < TW; i += blockDim.x) {
         for (unsigned mk = S.touched[i]; mk; mk &= mk - 1) S.cnt[(i << 5) + __ffs(mk) - 1] = 0;
         S.touched[i] = 0;
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
       for (int i = cs + tid; i < cend; i += blockDim.x) S.adjbits[(__ldg(Nv + i) - lo) >> 5] = 0;
       cv = cend;
       if (lane == 0 && nxt < v) atomicMin(&S.lo, max(hi, (nxt / CH) * CH));
-      __syncthreads();
+      block_sync();
     }
   }
 #pragma unroll

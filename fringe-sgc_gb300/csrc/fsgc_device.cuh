@@ -210,10 +210,10 @@ __host__ __device__ inline X128 nck_x(int n, int k) {
 }
 
 // ----------------------------------------------------------------------------
-// Block barrier for kernels whose warps may arrive with their lanes apart: the
-// form of barrier.sync without .aligned counts threads.  __syncthreads() (the
-// aligned form) counted such warps twice after long divergent loops, which let
-// the others through early.
+// The block barrier of every kernel here.  A warp may arrive with its lanes
+// apart (after a loop whose trip counts differ by lane, or a branch of lane 0):
+// the aligned form, which __syncthreads() is, is undefined then, while
+// barrier.sync without .aligned counts threads.
 __device__ __forceinline__ void block_sync() { asm volatile("barrier.sync 0;" ::: "memory"); }
 
 // ----------------------------------------------------------------------------

@@ -117,7 +117,7 @@ __device__ __forceinline__ long long block_excl_scan(long long x, long long* s_w
     if (lane >= o) inc += y;
   }
   if (lane == 31) s_warp[w] = inc;
-  __syncthreads();
+  block_sync();
   if (w == 0) {
     long long t = (lane < (int)(blockDim.x >> 5)) ? s_warp[lane] : 0;
     long long ti = t;
@@ -129,10 +129,10 @@ __device__ __forceinline__ long long block_excl_scan(long long x, long long* s_w
     if (lane < (int)(blockDim.x >> 5)) s_warp[lane] = ti - t;
     if (lane == 31) s_warp[32] = ti;
   }
-  __syncthreads();
+  block_sync();
   const long long r = s_warp[w] + inc - x;
   total = s_warp[32];
-  __syncthreads();
+  block_sync();
   return r;
 }
 

@@ -155,34 +155,33 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
     } else {
       total += acc;
     }
-    if (__syncthreads_or(d > kLinBlock)) {
-      for (int b = 0; b < kTPB / 32; b++) {
-        const int h = s_big[b];
-        if (h < 0) continue;
-        A p = A(0), q = A(0), a2 = A(0);
-        span(g.adj + g.off[h], g.deg[h], threadIdx.x, kTPB, p, q, a2);
-        const A pe = warp_excl(p), qe = same ? pe : warp_excl(q);
-        a2 += same ? p * pe : p * qe + q * pe;
-        if (lane == 31) {
-          s_p[warp] = pe + p;
-          s_q[warp] = qe + q;
+    block_sync();
+    for (int b = 0; b < kTPB / 32; b++) {
+      const int h = s_big[b];
+      if (h < 0) continue;
+      A p = A(0), q = A(0), a2 = A(0);
+      span(g.adj + g.off[h], g.deg[h], threadIdx.x, kTPB, p, q, a2);
+      const A pe = warp_excl(p), qe = same ? pe : warp_excl(q);
+      a2 += same ? p * pe : p * qe + q * pe;
+      if (lane == 31) {
+        s_p[warp] = pe + p;
+        s_q[warp] = qe + q;
+      }
+      block_sync();
+      if (threadIdx.x == 0) {
+        A ps = A(0), qs = A(0);
+        for (int w = 0; w < kTPB / 32; w++) {
+          a2 += same ? s_p[w] * ps : s_p[w] * qs + s_q[w] * ps;
+          ps += s_p[w];
+          qs += s_q[w];
         }
-        block_sync();
-        if (threadIdx.x == 0) {
-          A ps = A(0), qs = A(0);
-          for (int w = 0; w < kTPB / 32; w++) {
-            a2 += same ? s_p[w] * ps : s_p[w] * qs + s_q[w] * ps;
-            ps += s_p[w];
-            qs += s_q[w];
-          }
-        }
-        block_sync();
-        if (g.comp) {
-          a2 = warp_sum_a(a2);
-          if (lane == 0 && a2) slot_add(a2, g.comp_slots + g.comp[h]);
-        } else {
-          total += a2;
-        }
+      }
+      block_sync();
+      if (g.comp) {
+        a2 = warp_sum_a(a2);
+        if (lane == 0 && a2) slot_add(a2, g.comp_slots + g.comp[h]);
+      } else {
+        total += a2;
       }
     }
     block_sync();  // s_big is free again

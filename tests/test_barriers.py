@@ -1,0 +1,24 @@
+"""How the kernels use block barriers, read from their source (a missed or early
+barrier shows on a GPU only by chance): warps arrive with their lanes apart, so
+every barrier is the unaligned block_sync."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fringe-sgc_gb300", "csrc")
+
+
+def kernel_sources():
+    """(file name, text without comments) of every device source."""
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        with open(path) as f:
+            text = f.read()
+        text = re.sub(r"/\*.*?\*/", lambda m: "\n" * m.group().count("\n"), text, flags=re.S)
+        yield os.path.basename(path), re.sub(r"//[^\n]*", "", text)
+
+
+def test_barriers_take_warps_with_their_lanes_apart():
+    aligned = r"__syncthreads|__barrier_sync|\bbar\.(sync|red|arrive)|barrier\.[a-z.]*aligned"
+    for name, text in kernel_sources():
+        for i, line in enumerate(text.split("\n"), 1):
+            assert not re.search(aligned, line), f"{name}:{i}: {line.strip()}"
