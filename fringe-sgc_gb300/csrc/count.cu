@@ -594,6 +594,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
 #pragma unroll
   for (int q = 0; q < NP; q++) acc[q] = A(0);
   for (;;) {
+    block_sync();  // every warp has read S.v and, to leave the loop below, S.lo
     if (tid == 0) {
       S.v = atomicAdd(queue, 1);
       S.lo = 0;
@@ -602,10 +603,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wedge_chunk_kernel(GView g, Wedg
     const int v = S.v;
     if (v >= g.n) break;
     const int dv = g.deg[v];
-    if (dv < ws.lim || (BIG ? dv <= ws.small_max : dv > ws.small_max)) {
-      block_sync();
-      continue;
-    }
+    if (dv < ws.lim || (BIG ? dv <= ws.small_max : dv > ws.small_max)) continue;
     // counter layout: `bits` per counter, 2^lper counters per word, CH ids per chunk
     const int bits = BIG ? 32 : wedge_counter_bits(dv);
     const int lper = BIG ? 0 : (bits == 16 ? 1 : (bits == 8 ? 2 : 3));

@@ -22,3 +22,21 @@ def test_barriers_take_warps_with_their_lanes_apart():
     for name, text in kernel_sources():
         for i, line in enumerate(text.split("\n"), 1):
             assert not re.search(aligned, line), f"{name}:{i}: {line.strip()}"
+
+
+def test_shared_queue_items_are_replaced_behind_a_barrier():
+    """A block's thread 0 fetches the next queue item into shared memory that all
+    warps read, also in the condition by which they leave the last item's loop:
+    a barrier stands directly before it."""
+    found = 0
+    for name, text in kernel_sources():
+        lines = [line.strip() for line in text.split("\n") if line.strip()]
+        for i, line in enumerate(lines):
+            if not re.match(r"(S\.|s_)\w+ = atomicAdd\(queue\b", line):
+                continue
+            at = i - 1
+            while not re.match(r"if \((tid|threadIdx\.x) == 0\)", lines[at]):
+                at -= 1
+            assert at >= i - 2 and lines[at - 1] == "block_sync();", f"{name}: {lines[at - 1:i + 1]}"
+            found += 1
+    assert found >= 2
