@@ -1254,15 +1254,16 @@ int enqueue_rank_a(DevGraph& G, const GView& gv, const WedgeParams* pats, u64* c
       ord.np = 0;
       continue;
     }
-    // no shared fringe and none on one end: W does not depend on C
-    if (p.f_vw == 0 && std::min(p.f_v, p.f_w) == 0) continue;
+    const bool fits = std::is_same<A, u128>::value || binomials_fit(G.maxdeg, std::max(p.f_v, std::max(p.f_vw, p.f_w)));
+    // no shared fringe and none on one end: W does not depend on C, as long as
+    // no binomial wraps before its division
+    if (fits && p.f_vw == 0 && std::min(p.f_v, p.f_w) == 0) continue;
     RankSet rs;
     memset(&rs, 0, sizeof(rs));
     rs.np = 1;
     rs.w = p;
     rs.lim = p.lim;
     rs.slot[0] = slots[i];
-    const bool fits = std::is_same<A, u128>::value || binomials_fit(G.maxdeg, std::max(p.f_v, std::max(p.f_vw, p.f_w)));
     rs.form = pair_form(p, fits);
     rs.roles = !fits;  // the sum does not depend on which end is which unless a binomial wraps
     st = launch_rank_set<false, A>(r, rs, G, s, launches, work);
