@@ -673,10 +673,11 @@ static int ordered_supports(DevGraph& g, const GView& v, cudaStream_t s, uint64_
   const size_t words = sizeof(int) * (size_t)std::max(me, n);
   const int rank_bits = bits_for((unsigned)n - 1);
   size_t t1 = 0, t2 = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, t1, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
-                                  (int*)nullptr, n, 0, 32, s);
-  cub::DeviceRadixSort::SortPairs(nullptr, t2, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
-                                  (int*)nullptr, me, 0, rank_bits, s);
+  auto room = [&](size_t& bytes, int items, int bits) {
+    return cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
+                                           (int*)nullptr, items, 0, bits, s) == cudaSuccess;
+  };
+  if (!room(t1, n, 32) || !room(t2, me, rank_bits)) return done(FSGC_EUNSUPPORTED);
   const size_t tb = std::max(t1, t2);
   // a vertex left to the blocks has more than kSupSmall out-edges or kSupPiece in-edges
   const size_t pieces = (size_t)me / (kSupSmall + 1) + 2 * ((size_t)me / kSupPiece) + 2;
@@ -686,18 +687,19 @@ static int ordered_supports(DevGraph& g, const GView& v, cudaStream_t s, uint64_
       !get(&temp, tb))
     return done(FSGC_EUNSUPPORTED);
   const int vg = grid_for((long long)n + 1, kTPB, 16), eg = grid_for(me, kTPB, 16);
-  size_t tt = tb;
+  // every pass indexes with what the sort before it wrote
+  auto sort = [&](const int* values, int* out, int items, int bits) {
+    size_t tt = tb;
+    return cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, values, out, items, 0, bits, s) == cudaSuccess;
+  };
   degree_keys_kernel<<<vg, kTPB, 0, s>>>(v, k1, v1);
-  cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, v1, into, n, 0, bits_for((unsigned)g.maxdeg), s);
+  if (!sort(v1, into, n, bits_for((unsigned)g.maxdeg))) return done(FSGC_EUNSUPPORTED);
   rank_scatter_kernel<<<vg, kTPB, 0, s>>>(n, into, rank_of);
   upper_keys_kernel<<<eg, kTPB, 0, s>>>(v, me, rank_of, k1, v1);
-  tt = tb;
-  cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, v1, into, me, 0, rank_bits, s);
+  if (!sort(v1, into, me, rank_bits)) return done(FSGC_EUNSUPPORTED);
   into_starts_kernel<<<vg, kTPB, 0, s>>>(n, k2, me, start);
   lower_keys_kernel<<<eg, kTPB, 0, s>>>(v, me, into, k1);
-  tt = tb;
-  if (cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, into, slot, me, 0, rank_bits, s) != cudaSuccess)
-    return done(FSGC_EUNSUPPORTED);
+  if (!sort(into, slot, me, rank_bits)) return done(FSGC_EUNSUPPORTED);
   places_kernel<<<eg, kTPB, 0, s>>>(v, me, slot, rank_of, k1, v1);
   cudaMemsetAsync(sup, 0, sizeof(unsigned) * (size_t)me, s);
   cudaMemsetAsync(work, 0, sizeof(SupWork), s);

@@ -1302,14 +1302,16 @@ int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& 
   };
   const size_t big = (size_t)std::max(n + 1, m);
   auto get = [&](void** p, size_t bytes) { return cudaMallocAsync(p, bytes, s) == cudaSuccess; };
-  // scratch of both sorts
+  // scratch of the sorts and the scan
   size_t t1 = 0, t2 = 0, t3 = 0;
   const int rank_bits = bits_for((unsigned)n);
-  cub::DeviceRadixSort::SortPairs(nullptr, t1, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
-                                  (int*)nullptr, n, 0, 32, s);
-  cub::DeviceRadixSort::SortPairs(nullptr, t2, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
-                                  (int*)nullptr, m, 0, rank_bits, s);
-  cub::DeviceScan::ExclusiveSum(nullptr, t3, (const int*)nullptr, (int*)nullptr, n + 1, s);
+  auto room = [&](size_t& bytes, int items, int bits) {
+    return cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
+                                           (int*)nullptr, items, 0, bits, s) == cudaSuccess;
+  };
+  if (!room(t1, n, 32) || !room(t2, m, rank_bits) ||
+      cub::DeviceScan::ExclusiveSum(nullptr, t3, (const int*)nullptr, (int*)nullptr, n + 1, s) != cudaSuccess)
+    return drop(FSGC_ECUDA);
   const size_t tb = std::max(t1, std::max(t2, t3));
   if (!get((void**)&k1, sizeof(unsigned) * big) || !get((void**)&k2, sizeof(unsigned) * big) ||
       !get((void**)&v1, sizeof(int) * big) || !get((void**)&rank, sizeof(int) * (size_t)n) ||
@@ -1321,23 +1323,26 @@ int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& 
     return drop(FSGC_EUNSUPPORTED);  // no room: the count takes the path without this copy
   }
   const int vg = grid_for((long long)n + 1, kTPB, 16);
+  // every pass indexes with what the sort or scan before it wrote
+  auto sort = [&](int* out, int items, int bits) {
+    size_t tt = tb;
+    return cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, v1, out, items, 0, bits, s) == cudaSuccess;
+  };
   rank_degree_keys_kernel<<<vg, kTPB, 0, s>>>(gv, G.maxdeg, k1, v1);
-  size_t tt = tb;
-  cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, v1, G.oid, n, 0, bits_for((unsigned)G.maxdeg), s);
+  if (!sort(G.oid, n, bits_for((unsigned)G.maxdeg))) return drop(FSGC_ECUDA);
   *launches += 1;
   if (gv.comp) {
-    cudaMemcpyAsync(v1, G.oid, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, s);
+    if (cudaMemcpyAsync(v1, G.oid, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+      return drop(FSGC_ECUDA);
     rank_member_keys_kernel<<<vg, kTPB, 0, s>>>(gv, v1, k1);
-    tt = tb;
-    cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, v1, G.oid, n, 0, bits_for((unsigned)G.ngraphs), s);
+    if (!sort(G.oid, n, bits_for((unsigned)G.ngraphs))) return drop(FSGC_ECUDA);
     *launches += 1;
   }
   rank_assign_kernel<<<vg, kTPB, 0, s>>>(gv, G.oid, rank, G.rdeg);
-  tt = tb;
-  cub::DeviceScan::ExclusiveSum(temp, tt, G.rdeg, G.roff, n + 1, s);
+  size_t tt = tb;
+  if (cub::DeviceScan::ExclusiveSum(temp, tt, G.rdeg, G.roff, n + 1, s) != cudaSuccess) return drop(FSGC_ECUDA);
   rank_entries_kernel<<<grid_for((long long)n * 32, kTPB, 16), kTPB, 0, s>>>(gv, G.oid, rank, G.roff, k1, v1);
-  tt = tb;
-  cub::DeviceRadixSort::SortPairs(temp, tt, k1, k2, v1, G.radj, m, 0, rank_bits, s);
+  if (!sort(G.radj, m, rank_bits)) return drop(FSGC_ECUDA);
   *launches += 2;
   // boundary table of the long lists (ordinary graphs; a packed graph's members
   // span few chunks), at most 256 MiB
