@@ -1235,6 +1235,11 @@ void fsgc_wedge_formula_host(int dx, int dy, int adj, int f_x, int f_xy, int f_y
   }
 }
 
+// The rule by which the loader finds edge supports through lists in rank order.
+int fsgc_supports_ordered_host(long long edges, int n, unsigned long long squares) {
+  return fsgc::supports_ordered(edges, n, squares) ? 1 : 0;
+}
+
 unsigned long long fsgc_div_small_host(unsigned long long x, unsigned d) {
   if (d < 2 || d >= (unsigned)fsgc::kMaxDiv) return 0;
   return fsgc::div_magic(x, fsgc::make_div_magic(d));

@@ -110,6 +110,10 @@ struct DevWork {
   fsgc_tuning tune = {2048, 16, 8192, 96, 8};
 };
 constexpr int kErrWord = 10;
+// Items that a kernel may walk with 32-bit indices: a grid-stride step (at most 16
+// blocks of 256 on each of up to 1,024 SMs) or a piece beyond the last one still
+// fits an int.
+constexpr int kMaxItems32 = 0x7fffffff - (1 << 22);
 // Wedge pairs in rank order from this many list entries: RMAT with 21,000 entries
 // counts in 0.11 ms either way, with 45,000 in 0.09 instead of 0.16 ms; below,
 // the copy only costs (pattern graphs, counted in themselves, stay there too).
@@ -128,6 +132,7 @@ bool matching_order_valid(const fsgc_matching_order& mo);
 // Entry points implemented in prep.cu / count.cu.
 int graph_degrees(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_scratch_u64);
 int prepare_graph(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_scratch_u64);
+bool supports_ordered(long long me, int n, u64 squares);  // prep.cu: the rule
 int ensure_vertex_triangles(DevGraph& g, cudaStream_t s, uint64_t* launches);
 int ensure_entry_supports(DevGraph& g, cudaStream_t s, uint64_t* launches);
 void upload_div_magic();

@@ -609,6 +609,12 @@ int g_sms = 0;
 
 }  // namespace
 
+// Whether the supports of `me` oriented edges between n vertices, `squares` the
+// sum of the squared out-degrees, are found through lists in rank order.
+bool supports_ordered(long long me, int n, u64 squares) {
+  return me >= kOrderedMin && me <= kMaxItems32 && n <= kMaxItems32 && squares >= (u64)kOrderedSquares * (u64)me;
+}
+
 int sm_count() {
   if (g_sms == 0) {
     int dev = 0;
@@ -652,10 +658,9 @@ int graph_degrees(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_u64) {
 }
 
 // Supports through lists in rank order; FSGC_EUNSUPPORTED, with nothing added,
-// beyond 32-bit positions or when there is no room.
+// when there is no room.  32-bit positions (supports_ordered).
 static int ordered_supports(DevGraph& g, const GView& v, cudaStream_t s, uint64_t* launches, u64* d_tri) {
   const int n = g.n;
-  if (g.m / 2 > 0x7fffff00LL || n > 0x7fffff00) return FSGC_EUNSUPPORTED;
   const int me = (int)(g.m / 2);
   auto bits_for = [](unsigned x) { int b = 1; while (b < 32 && x >> b) b++; return b; };
   unsigned *k1 = nullptr, *k2 = nullptr, *sup = nullptr;
@@ -750,7 +755,7 @@ int prepare_graph(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_u64) {
     u64 squares = 0;
     FSGC_TRY(cudaMemcpyAsync(&squares, d_stats + 4, sizeof(u64), cudaMemcpyDeviceToHost, s));
     FSGC_TRY(cudaStreamSynchronize(s));
-    ordered = squares >= (u64)kOrderedSquares * (u64)me && ordered_supports(g, v, s, launches, d_tri) == FSGC_OK;
+    ordered = supports_ordered(me, n, squares) && ordered_supports(g, v, s, launches, d_tri) == FSGC_OK;
   }
   if (me > 0 && !ordered) {
     triangle_support_kernel<<<grid_for(me, kTPB, 8), kTPB, 0, s>>>(v, g.osup, d_tri);
