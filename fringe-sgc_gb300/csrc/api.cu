@@ -147,6 +147,10 @@ int ensure_events(fsgc_ctx* c, size_t n) {
   return FSGC_OK;
 }
 
+// Vertex counts that the kernels' 32-bit vertex loops can walk.
+#define FSGC_CHECK_VERTICES(n) \
+  if ((n) > fsgc::kMaxItems32) return fail(c, FSGC_EUNSUPPORTED, "more than %d vertices", fsgc::kMaxItems32)
+
 // Upload a host CSR (64-bit offsets) as a new DevGraph.
 int upload_graph(fsgc_ctx* c, int n, long long m, const long long* off, const int* adj, bool device_src,
                  DevGraph** out) {
@@ -561,6 +565,7 @@ int fsgc_ctx_synchronize(fsgc_ctx* c) {
 
 int fsgc_graph_from_csr(fsgc_ctx* c, int n, int64_t m, const int64_t* nindex, const int32_t* nlist, int* gid) {
   if (!c || !gid || n < 1 || m < 0 || !nindex || (m > 0 && !nlist)) return fail(c, FSGC_EINVAL, "bad graph arguments");
+  FSGC_CHECK_VERTICES(n);
   if (nindex[0] != 0 || nindex[n] != m) return fail(c, FSGC_EINVAL, "offsets must start at 0 and end at m");
   for (int v = 0; v < n; v++)
     if (nindex[v + 1] < nindex[v]) return fail(c, FSGC_EINVAL, "offsets decrease at vertex %d", v);
@@ -577,6 +582,7 @@ int fsgc_graph_from_csr(fsgc_ctx* c, int n, int64_t m, const int64_t* nindex, co
 
 int fsgc_graph_from_csr32(fsgc_ctx* c, int n, int m, const int32_t* nindex, const int32_t* nlist, int* gid) {
   if (!c || n < 1 || m < 0 || !nindex) return fail(c, FSGC_EINVAL, "bad graph arguments");
+  FSGC_CHECK_VERTICES(n);
   std::vector<int64_t> off((size_t)n + 1);
   for (int v = 0; v <= n; v++) off[v] = nindex[v];
   return fsgc_graph_from_csr(c, n, m, off.data(), nlist, gid);
@@ -585,6 +591,7 @@ int fsgc_graph_from_csr32(fsgc_ctx* c, int n, int m, const int32_t* nindex, cons
 int fsgc_graph_from_device_csr(fsgc_ctx* c, int n, int64_t m, const int64_t* d_nindex, const int32_t* d_nlist,
                                int* gid) {
   if (!c || !gid || n < 1 || m < 0 || !d_nindex || (m > 0 && !d_nlist)) return fail(c, FSGC_EINVAL, "bad graph arguments");
+  FSGC_CHECK_VERTICES(n);
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
   DevGraph* g = nullptr;
@@ -597,6 +604,7 @@ int fsgc_graph_from_device_csr(fsgc_ctx* c, int n, int64_t m, const int64_t* d_n
 
 int fsgc_graph_from_edges(fsgc_ctx* c, int n, int64_t nedges, const int32_t* pairs, int pairs_on_device, int* gid) {
   if (!c || !gid || n < 1 || nedges < 0 || (nedges > 0 && !pairs)) return fail(c, FSGC_EINVAL, "bad edge-list arguments");
+  FSGC_CHECK_VERTICES(n);
   std::lock_guard<std::mutex> lk(c->mu);
   cudaSetDevice(c->device);
   const int* d_pairs = pairs;
@@ -679,6 +687,7 @@ int fsgc_graph_from_packed_csr(fsgc_ctx* c, int n, int64_t m, const int64_t* nin
                                int ngraphs, const int32_t* vstart, int* gid) {
   if (!c || !gid || n < 1 || m < 0 || !nindex || (m > 0 && !nlist) || ngraphs < 1 || !vstart)
     return fail(c, FSGC_EINVAL, "bad packed graph arguments");
+  FSGC_CHECK_VERTICES(n);
   if (vstart[0] != 0 || vstart[ngraphs] != n) return fail(c, FSGC_EINVAL, "member ranges must cover [0, n)");
   if (nindex[0] != 0 || nindex[n] != m) return fail(c, FSGC_EINVAL, "offsets must start at 0 and end at m");
   std::vector<int> comp((size_t)n);

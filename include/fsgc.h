@@ -159,7 +159,9 @@ int fsgc_ctx_get_tuning(fsgc_ctx* ctx, fsgc_tuning* out);
 
 /* ---- resident graphs (CSR upload + loader: src/fringeCount.cu:2286-2297) ---- */
 
-/* Uploads a host CSR (offsets 64-bit) and prepares it for counting. */
+/* Uploads a host CSR (offsets 64-bit) and prepares it for counting.  Graphs of more than
+ * 2^31 - 1 - 2^22 vertices are refused (FSGC_EUNSUPPORTED), here and by the calls below:
+ * the kernels walk the vertices with 32-bit indices. */
 int fsgc_graph_from_csr(fsgc_ctx* ctx, int n, int64_t m, const int64_t* nindex, const int32_t* nlist, int* gid);
 /* Same with the reference's int32 offsets (ECLgraph layout). */
 int fsgc_graph_from_csr32(fsgc_ctx* ctx, int n, int m, const int32_t* nindex, const int32_t* nlist, int* gid);
