@@ -110,13 +110,7 @@ void free_graph(DevGraph* g) {
   cudaFree(g->ctab_pos);
   cudaFree(g->wide);
   cudaFree(g->bits);
-  cudaFree(g->roff);
-  cudaFree(g->radj);
-  cudaFree(g->rdeg);
-  cudaFree(g->oid);
-  cudaFree(g->rrev);
-  cudaFree(g->radj16);
-  cudaFree(g->rtab);
+  fsgc::free_rank_order(*g);
   cudaFree(g->comp);
   cudaFree(g->comp_relabel);
   delete g;
@@ -361,7 +355,8 @@ int count_tasks(fsgc_ctx* c, const fsgc_task* tasks, int nt, fsgc_result* res) {
   return FSGC_OK;
 }
 
-// Captured pattern-set launches of graph `gid` (all graphs when gid < 0).
+// Captured pattern-set launches of graph `gid` (all graphs when gid < 0); its
+// sets start over with a direct call, which builds what the graph lacks.
 void drop_set_graphs(fsgc_ctx* c, int gid) {
   for (auto it = c->set_graphs.begin(); it != c->set_graphs.end();) {
     if (gid < 0 || it->second.gid == gid) {
@@ -371,7 +366,10 @@ void drop_set_graphs(fsgc_ctx* c, int gid) {
       ++it;
     }
   }
-  if (gid < 0) c->set_seen.clear();
+  for (auto it = c->set_seen.begin(); it != c->set_seen.end();) {
+    if (gid < 0 || memcmp(it->first.data(), &gid, sizeof(gid)) == 0) it = c->set_seen.erase(it);
+    else ++it;
+  }
 }
 
 }  // namespace
@@ -831,6 +829,28 @@ int fsgc_graph_prepare_all(fsgc_ctx* c, int gid) {
   const int st = fsgc::prepare_all(*g, c->stream, &c->launches, c->work);
   if (st != FSGC_OK) return fail(c, st, "graph preparation failed: %s", cudaGetErrorString(cudaGetLastError()));
   return FSGC_OK;
+}
+
+int fsgc_graph_lean(fsgc_ctx* c, int gid, int on) {
+  if (!c) return FSGC_EINVAL;
+  std::lock_guard<std::mutex> lk(c->mu);
+  cudaSetDevice(c->device);
+  DevGraph* g = find_graph(c, gid);
+  if (!g) return fail(c, FSGC_ENOTFOUND, "unknown graph %d", gid);
+  if (g->lean == (on != 0)) return FSGC_OK;
+  // lanes may be counting on the structures, captured sets hold their addresses
+  CK(cudaDeviceSynchronize(), "counts in flight");
+  drop_set_graphs(c, gid);
+  g->lean = on != 0;
+  if (on) fsgc::free_fast_structures(*g);
+  return FSGC_OK;
+}
+
+size_t fsgc_graph_fast_bytes(fsgc_ctx* c, int gid) {
+  if (!c) return 0;
+  std::lock_guard<std::mutex> lk(c->mu);
+  DevGraph* g = find_graph(c, gid);
+  return g ? fsgc::fast_structure_bytes(*g) : 0;
 }
 
 int fsgc_graph_info_get(fsgc_ctx* c, int gid, fsgc_graph_info* out) {

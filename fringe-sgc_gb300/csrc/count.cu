@@ -1444,14 +1444,15 @@ __global__ void bit_matrix_kernel(GView g, int words, unsigned* __restrict__ mat
 }
 
 int bit_matrix_words(int n) { return ((n + 31) / 32 + 3) & ~3; }
+size_t bit_matrix_bytes(const DevGraph& G) { return sizeof(unsigned) * (size_t)G.n * bit_matrix_words(G.n); }
 
 // The adjacency bit matrix of a small graph, once per graph (at most 2 MiB).
 // FSGC_EUNSUPPORTED when the graph is larger or there was no room for it: the
 // caller takes the lists.
 int ensure_bit_matrix(DevGraph& G, cudaStream_t s, uint64_t* launches) {
   if (G.bits) return FSGC_OK;
-  if (G.bits_failed || G.n > kBitsMaxN) return FSGC_EUNSUPPORTED;
-  const size_t bytes = sizeof(unsigned) * (size_t)G.n * bit_matrix_words(G.n);
+  if (G.lean || G.bits_failed || G.n > kBitsMaxN) return FSGC_EUNSUPPORTED;
+  const size_t bytes = bit_matrix_bytes(G);
   if (cudaMallocAsync((void**)&G.bits, bytes, s) != cudaSuccess) {
     cudaGetLastError();
     G.bits = nullptr;
@@ -1823,6 +1824,15 @@ int check_tuning(const fsgc_tuning& t) {
   return ok ? FSGC_OK : FSGC_EINVAL;
 }
 
+size_t fast_structure_bytes(const DevGraph& G) { return G.rank_bytes + (G.bits ? bit_matrix_bytes(G) : 0); }
+
+void free_fast_structures(DevGraph& G) {
+  if (G.bits) G.bytes -= bit_matrix_bytes(G);
+  free_rank_order(G);
+  cudaFree(G.bits);
+  G.bits = nullptr;
+}
+
 int prepare_for_count(const fsgc_matching_order& mo, DevGraph& G, cudaStream_t s, uint64_t* launches,
                       DevWork& work) {
   if (mo.nodes < 2) return FSGC_OK;
@@ -1849,12 +1859,14 @@ int prepare_for_count(const fsgc_matching_order& mo, DevGraph& G, cudaStream_t s
   return cudaStreamSynchronize(s) == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
 
+// The chunk table is for graphs without a copy in rank order: beside one, only
+// exact counts beyond its bound read it, and they build it.
 int prepare_all(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) {
   int st = prepare_graph(G, s, launches, work.small);
-  if (st == FSGC_OK && G.ngraphs == 0) st = ensure_chunk_table(G, s, launches, work.small + 9);
   if (st == FSGC_OK) {
     st = ensure_rank_order(G, s, launches, work);
-    if (st == FSGC_EUNSUPPORTED) st = FSGC_OK;  // counted another way
+    if (st == FSGC_EUNSUPPORTED)  // counted another way
+      st = G.ngraphs == 0 ? ensure_chunk_table(G, s, launches, work.small + 9) : FSGC_OK;
   }
   if (st == FSGC_OK) st = ensure_vertex_triangles(G, s, launches);
   if (st == FSGC_OK && G.ngraphs == 0) st = ensure_entry_supports(G, s, launches);

@@ -68,9 +68,11 @@ struct DevGraph {
   int* rrev = nullptr;  // per list entry (v, u): entries of N(u) up to v
   int* rtab = nullptr;  // boundary table of the first rrows lists, rK columns
   int rrows = 0, rK = 0;
+  size_t rank_bytes = 0;     // of the copy (0: there is none)
   bool rank_failed = false;  // no room for the copy: not tried again
   unsigned* bits = nullptr;  // lazily: adjacency bit matrix of a small graph (general cores)
   bool bits_failed = false;  // no room for it: not tried again
+  bool lean = false;  // neither of the two is built: counts take the paths without them
   // the reference's degree-relabel gate for the triangle core
   // (src/fringeCount.cu:1237, 1342-1344): vertex roles follow (deg, id) order
   // when it fires, vertex ids otherwise
@@ -202,6 +204,7 @@ inline bool wedge_rank_size_ok(const DevGraph& G) {
 // the copy, or (exact) the total is not bounded below 2^128: nothing is
 // enqueued then and the caller counts another way.
 int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work);
+void free_rank_order(DevGraph& G);  // no work that reads it in flight
 int enqueue_wedge_rank(DevGraph& G, const GView& gv, const WedgeParams* pats, u64* const* slots, int np, bool exact,
                        cudaStream_t s, uint64_t* launches, DevWork& work);
 size_t wedge_rank_scratch(const DevGraph& G);  // work-arena bytes (cursors of hub owners)
@@ -231,6 +234,10 @@ int csr_from_device_edges(int n, long long E, const int* d_pairs, cudaStream_t s
                           long long* m_out, u64* d_small);
 // Builds every per-graph structure any count could need, synchronously.
 int prepare_all(DevGraph& g, cudaStream_t s, uint64_t* launches, DevWork& work);
+// What DevGraph::lean leaves out: its bytes, and freeing it (nothing that reads it
+// is in flight).
+size_t fast_structure_bytes(const DevGraph& g);
+void free_fast_structures(DevGraph& g);
 // Scratch-arena bytes a count of `mo` on the prepared graph `g` grows to.
 size_t count_scratch_bytes(const fsgc_matching_order& mo, const DevGraph& g, const fsgc_tuning& t);
 // FSGC_EINVAL unless every field of `t` is in its documented range.

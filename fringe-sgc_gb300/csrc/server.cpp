@@ -15,10 +15,13 @@
 // re-run one query at a time, so that a bad query fails alone, and when a
 // count fails inside a batch the queries after it are re-run one at a time.
 // Registering a graph builds every derived structure any count could need
-// (orientation, supports, chunk table, per-vertex triangles, per-entry
-// supports), so no query builds one under the context lock while other lanes
-// wait, and the graph's device bytes count against the budget for as long as
-// it is registered, beside the lanes' work arenas.  Latency is
+// (orientation, supports, the copy in rank order or the chunk table, per-vertex
+// triangles, per-entry supports, the bit matrix of a small graph), so no query
+// builds one under the context lock while other lanes wait, and the graph's
+// device bytes count against the budget for as long as it is registered, beside
+// the lanes' work arenas.  The copy and the bit matrix only make counts faster:
+// where a graph or a query fits the budget without them alone, registered graphs
+// give them up, the one at hand first.  Latency is
 // submission to completion.  Results are cached by (graph, matching-order
 // bytes): resident graphs never change and graph ids are never reused, so a
 // repeated query completes at submission without device work.
@@ -35,6 +38,12 @@
 #include <vector>
 
 #include "fsgc.h"
+
+// Absent where the loop is linked with stand-ins for the device calls.
+extern "C" {
+__attribute__((weak)) int fsgc_graph_lean(fsgc_ctx* ctx, int gid, int on);
+__attribute__((weak)) size_t fsgc_graph_fast_bytes(fsgc_ctx* ctx, int gid);
+}
 
 namespace {
 
@@ -74,7 +83,12 @@ struct fsgc_server {
   bool stop = false;
   std::vector<LaneSlot> lanes;
   std::vector<std::thread> workers;
-  std::map<int, int> graphs;  // registered graph ids
+  struct Resident {
+    size_t bytes = 0;
+    bool lean = false;  // made so by this server
+  };
+  std::mutex graph_mu;  // held while graphs are registered or made lean; taken before mu
+  std::map<int, Resident> graphs;  // by graph id
   std::map<std::pair<int, std::string>, fsgc_result> cache;  // completed counts
   static constexpr size_t kCacheCap = 1 << 16;               // entries; cleared when full
   uint64_t cache_hits = 0;
@@ -217,6 +231,43 @@ void worker_loop(fsgc_server* s, int li) {
   }
 }
 
+int graph_bytes(fsgc_server* s, int gid, size_t* bytes) {
+  fsgc_graph_info info;
+  const int st = fsgc_graph_info_get(s->ctx, gid, &info);
+  if (st == FSGC_OK) *bytes = (size_t)std::max<int64_t>(0, info.device_bytes);
+  return st;
+}
+
+// Brings `used()` down to the budget by making registered graphs lean, in the
+// order of their ids and no more of them than it takes; false, with none
+// touched, where all of them would not do (graph_mu held, mu not).
+template <class F>
+bool make_room(fsgc_server* s, F used) {
+  if (!fsgc_graph_lean || !fsgc_graph_fast_bytes) return false;
+  auto over = [&](size_t spare) {
+    std::lock_guard<std::mutex> lk(s->mu);
+    return used() > s->budget + spare;
+  };
+  size_t spare = 0;
+  for (auto& g : s->graphs)  // only changed under graph_mu
+    if (!g.second.lean) spare += fsgc_graph_fast_bytes(s->ctx, g.first);
+  if (over(spare)) return false;
+  for (auto& g : s->graphs) {
+    if (!over(0)) return true;
+    if (g.second.lean || fsgc_graph_fast_bytes(s->ctx, g.first) == 0) continue;
+    size_t bytes = 0;
+    int st = fsgc_graph_lean(s->ctx, g.first, 1);
+    if (st == FSGC_OK) st = fsgc_graph_prepare_all(s->ctx, g.first);
+    if (st == FSGC_OK) st = graph_bytes(s, g.first, &bytes);
+    std::lock_guard<std::mutex> lk(s->mu);
+    g.second.lean = true;
+    if (st != FSGC_OK) continue;  // released since, or no room for its table: the charge stays
+    s->resident = s->resident - g.second.bytes + bytes;
+    g.second.bytes = bytes;
+  }
+  return !over(0);
+}
+
 double percentile(std::vector<double> v, double p) {
   if (v.empty()) return 0;
   std::sort(v.begin(), v.end());
@@ -261,23 +312,43 @@ void fsgc_server_destroy(fsgc_server* s) {
   for (auto& w : s->workers)
     if (w.joinable()) w.join();
   for (auto& l : s->lanes) fsgc_lane_destroy(l.lane);
+  for (auto& g : s->graphs)
+    if (g.second.lean) fsgc_graph_lean(s->ctx, g.first, 0);
   delete s;
 }
 
 int fsgc_server_add_graph(fsgc_server* s, int gid) {
   if (!s) return FSGC_EINVAL;
-  int st = fsgc_graph_prepare_all(s->ctx, gid);
+  std::lock_guard<std::mutex> reg(s->graph_mu);
+  size_t bytes = 0;
+  int st = graph_bytes(s, gid, &bytes);  // a released graph is no longer known
   if (st != FSGC_OK) return st;
-  fsgc_graph_info info;
-  st = fsgc_graph_info_get(s->ctx, gid, &info);
+  {
+    std::lock_guard<std::mutex> lk(s->mu);
+    if (s->graphs.count(gid)) return FSGC_OK;
+  }
+  st = fsgc_graph_prepare_all(s->ctx, gid);
+  if (st == FSGC_OK) st = graph_bytes(s, gid, &bytes);
   if (st != FSGC_OK) return st;
-  std::lock_guard<std::mutex> lk(s->mu);
-  if (s->graphs.count(gid)) return FSGC_OK;
-  const size_t bytes = (size_t)std::max<int64_t>(0, info.device_bytes);
-  if (s->resident + s->held_total + bytes > s->budget) return FSGC_EBUSY;  // does not fit beside what is there
-  s->resident += bytes;
-  s->graphs[gid] = 1;
-  return FSGC_OK;
+  auto take = [&](bool lean) {
+    std::lock_guard<std::mutex> lk(s->mu);
+    if (s->resident + s->held_total + bytes > s->budget) return false;
+    s->resident += bytes;
+    s->graphs[gid] = fsgc_server::Resident{bytes, lean};
+    return true;
+  };
+  if (take(false)) return FSGC_OK;
+  // without what only makes its own counts faster, then the others'
+  const bool lean = fsgc_graph_lean && fsgc_graph_fast_bytes && fsgc_graph_fast_bytes(s->ctx, gid) > 0;
+  if (lean) {
+    st = fsgc_graph_lean(s->ctx, gid, 1);
+    if (st == FSGC_OK) st = fsgc_graph_prepare_all(s->ctx, gid);
+    if (st == FSGC_OK) st = graph_bytes(s, gid, &bytes);
+    if (st == FSGC_OK && take(true)) return FSGC_OK;
+  }
+  if (st == FSGC_OK && make_room(s, [&] { return s->resident + s->held_total + bytes; }) && take(lean)) return FSGC_OK;
+  if (lean) fsgc_graph_lean(s->ctx, gid, 0);
+  return st != FSGC_OK ? st : FSGC_EBUSY;  // does not fit beside what is there
 }
 
 int fsgc_server_submit(fsgc_server* s, int gid, const fsgc_matching_order* mo, uint64_t* ticket) {
@@ -317,9 +388,17 @@ int fsgc_server_submit(fsgc_server* s, int gid, const fsgc_matching_order* mo, u
   size_t fp = 0;
   const int st = fsgc_task_footprint(s->ctx, &task, &fp);
   if (st != FSGC_OK) return st;
+  bool fits;
+  {
+    std::lock_guard<std::mutex> lk(s->mu);
+    fits = s->resident + fp <= s->budget;
+  }
+  if (!fits) {
+    // can never be admitted beside the registered graphs as they are
+    std::lock_guard<std::mutex> reg(s->graph_mu);
+    if (!make_room(s, [&] { return s->resident + fp; })) return FSGC_EBUSY;
+  }
   std::lock_guard<std::mutex> lk(s->mu);
-  // can never be admitted beside the registered graphs
-  if (s->resident + fp > s->budget) return FSGC_EBUSY;
   Query q;
   q.ticket = s->next_ticket++;
   q.gid = gid;

@@ -1280,7 +1280,7 @@ bool binomials_fit(int maxdeg, int k) {
 
 int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) {
   if (G.radj) return FSGC_OK;
-  if (G.rank_failed || !wedge_rank_size_ok(G)) return FSGC_EUNSUPPORTED;
+  if (G.lean || G.rank_failed || !wedge_rank_size_ok(G)) return FSGC_EUNSUPPORTED;
   const int n = G.n;
   const int m = (int)G.m;
   const GView gv = G.view();
@@ -1371,9 +1371,20 @@ int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& 
   rank_reverse_kernel<<<grid_for((long long)n * 32, kTPB, 16), kTPB, 0, s>>>(G.roff, G.radj, G.rdeg, n, G.rtab, G.rrows,
                                                                             G.rK, G.rrev);
   *launches += 2;
-  G.bytes += sizeof(int) * ((size_t)3 * n + 2 + (size_t)2 * m + (size_t)G.rrows * G.rK) + sizeof(short) * (size_t)m;
+  G.rank_bytes = sizeof(int) * ((size_t)3 * n + 2 + (size_t)2 * m + (size_t)G.rrows * G.rK) + sizeof(short) * (size_t)m;
+  G.bytes += G.rank_bytes;
   drop(FSGC_OK);
   return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
+}
+
+void free_rank_order(DevGraph& G) {
+  for (void* p : {(void*)G.roff, (void*)G.radj, (void*)G.rdeg, (void*)G.oid, (void*)G.rrev, (void*)G.radj16, (void*)G.rtab})
+    cudaFree(p);
+  G.roff = G.radj = G.rdeg = G.oid = G.rrev = G.rtab = nullptr;
+  G.radj16 = nullptr;
+  G.rrows = G.rK = 0;
+  G.bytes -= G.rank_bytes;
+  G.rank_bytes = 0;
 }
 
 size_t wedge_rank_scratch(const DevGraph& G) {

@@ -118,6 +118,8 @@ def lib():
             "fsgc_graph_from_edges": (I, [P, I, I64, P, I, C.POINTER(C.c_int)]),
             "fsgc_graph_copy_csr": (I, [P, I, P, P]),
             "fsgc_graph_prepare_all": (I, [P, I]),
+            "fsgc_graph_lean": (I, [P, I, I]),
+            "fsgc_graph_fast_bytes": (C.c_size_t, [P, I]),
             "fsgc_tuning_default": (I, [C.POINTER(Tuning)]),
             "fsgc_ctx_set_tuning": (I, [P, C.POINTER(Tuning)]),
             "fsgc_ctx_get_tuning": (I, [P, C.POINTER(Tuning)]),
@@ -400,6 +402,11 @@ class Context:
 
     def prepare_all(self, gid):
         _check(lib().fsgc_graph_prepare_all(self.ptr, gid), "graph_prepare_all", self.ptr)
+
+    def lean(self, gid, on=True):
+        """Gives back the structures that only make counts faster, and builds them
+        no more until called with on=False."""
+        _check(lib().fsgc_graph_lean(self.ptr, gid, 1 if on else 0), "graph_lean", self.ptr)
 
     def load_egr(self, path):
         gid = C.c_int()

@@ -185,9 +185,17 @@ int fsgc_graph_release(fsgc_ctx* ctx, int gid);
  * worklist builders, src/fringeCount.cu:1221-1288, 617-663, 1167-1218). */
 int fsgc_graph_prepare(fsgc_ctx* ctx, int gid);
 /* Builds, now, every derived structure any count on this graph could need:
- * the passes above plus the wedge core's chunk table, the per-vertex triangle
- * counts and the per-entry supports (their bytes show in device_bytes). */
+ * the passes above plus the wedge core's copy in rank order (its chunk table
+ * where there is none), the per-vertex triangle counts, the per-entry supports
+ * and a small graph's bit matrix (their bytes show in device_bytes). */
 int fsgc_graph_prepare_all(fsgc_ctx* ctx, int gid);
+/* on != 0: gives back the two that only make counts faster, the copy in rank
+ * order (10 bytes a list entry and up to 256 MiB) and the bit matrix, after what
+ * is running has ended, and builds them no more; on == 0: the next count that
+ * uses them builds them again.  Counts are the same either way. */
+int fsgc_graph_lean(fsgc_ctx* ctx, int gid, int on);
+/* Device bytes that those two take now (0 for an unknown graph). */
+size_t fsgc_graph_fast_bytes(fsgc_ctx* ctx, int gid);
 
 typedef struct fsgc_graph_info {
   int32_t n;
@@ -292,6 +300,8 @@ int fsgc_task_footprint(fsgc_ctx* ctx, const fsgc_task* task, size_t* bytes);
  * fsgc_server_add_graph, which builds every derived structure a count could
  * need (fsgc_graph_prepare_all) and counts the graph's device bytes against
  * `memory_budget` while it is registered (FSGC_EBUSY when it does not fit).
+ * Where a graph or a query fits only without them, registered graphs give up the
+ * structures that fsgc_graph_lean names, for as long as the server exists.
  * Submitted queries wait in arrival order.  Whenever a lane is free, its
  * worker admits queries from the head of the queue (at most `max_batch`)
  * while the registered graphs and the lanes' work arenas, with this batch's
