@@ -516,6 +516,17 @@ size_t shape_block(TriLaunch& p, int kmax, int warps, size_t smem) {
   return bytes;
 }
 
+constexpr size_t kWideSmem = 111 * 1024;
+
+// Rows of the triangle core that do not fit in a wide block's shared memory (each
+// with at most one pad word) go to the arena: unpadded, at most 8 GiB in all.
+bool rows_fit(const DevGraph& G, int rows) { return G.max_bitmap_words + G.max_outdeg <= rows; }
+long long arena_words(const DevGraph& G) { return std::max(1LL, G.max_bitmap_words); }
+int arena_blocks(const DevGraph& G) {
+  const size_t per = sizeof(unsigned) * (size_t)arena_words(G);
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)2 * sm_count(), ((size_t)8 << 30) / per));
+}
+
 template <int MODE, int NT, class A>
 int launch_blocks(DevGraph& G, const GView& gv, const TriLaunch& p, size_t smem, u64* slot, cudaStream_t s, int blocks,
                   uint64_t* launches, DevWork& work) {
@@ -535,28 +546,31 @@ int launch_mode(DevGraph& G, const GView& gv, TriLaunch p, u64* slot, cudaStream
   const int kmax = (int)std::max(1LL, G.max_outdeg);
   TriLaunch n = p;
   const size_t nsmem = shape_block(n, std::min(kmax, kTriNarrowK), kNarrow / 32, 35 * 1024);
-  const size_t wsmem = shape_block(p, kmax, kWide / 32, 111 * 1024);
+  const size_t wsmem = shape_block(p, kmax, kWide / 32, kWideSmem);
   if (n.rows < kTriNarrowRows) return FSGC_EINVAL;  // the block holds what triangle_wide leaves to it
   n.items = G.n;
   p.list = G.wide;
   p.items = G.nwide;
   int st = launch_blocks<MODE, kNarrow, A>(G, gv, n, nsmem, slot, s, 6 * sm_count(), launches, work);
   if (st != FSGC_OK || G.nwide == 0) return st;
-  // row words, each row with at most one pad word
-  const long long words = MODE % 3 == 0 ? G.max_bitmap_words : (long long)kmax * ((kmax + 31) / 32);
   int blocks = 2 * sm_count();
-  if (MODE % 3 == 0 && words + kmax > p.rows) {
-    // rows that do not fit in shared memory: in the arena, at most 8 GiB of it
-    p.gstride = std::max(1LL, words);
-    const size_t per = sizeof(unsigned) * (size_t)p.gstride;
-    blocks = (int)std::max<size_t>(1, std::min<size_t>((size_t)blocks, ((size_t)8 << 30) / per));
-    st = ensure_plain_scratch(work.tri, per * (size_t)blocks, s);
+  if (MODE % 3 == 0 && !rows_fit(G, p.rows)) {
+    blocks = arena_blocks(G);
+    p.gstride = arena_words(G);
+    st = ensure_plain_scratch(work.tri, triangle_scratch(G), s);
     if (st != FSGC_OK) return st;
   }
   return launch_blocks<MODE, kWide, A>(G, gv, p, wsmem, slot, s, blocks, launches, work);
 }
 
 }  // namespace
+
+size_t triangle_scratch(const DevGraph& G) {
+  TriLaunch p;
+  shape_block(p, (int)std::max(1LL, G.max_outdeg), kWide / 32, kWideSmem);
+  if (G.nwide == 0 || rows_fit(G, p.rows)) return 0;
+  return sizeof(unsigned) * (size_t)arena_words(G) * (size_t)arena_blocks(G);
+}
 
 bool triangle_by_tables(const DevGraph& G) { return G.max_outdeg <= kMaxOut && G.m / 2 > 0; }
 
