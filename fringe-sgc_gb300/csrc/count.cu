@@ -1802,12 +1802,7 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
   }
   const bool clique = (f[IUVW] == 1) && (f[IUV] + f[IUW] + f[IVW] == 0) &&
                       ((f[IU] == 0) + (f[IV] == 0) + (f[IW] == 0) >= 2);
-  if (!clique && triangle_by_tables(G)) {
-    // rows of vertices that do not fit in shared memory: at most three blocks'
-    // worth per SM and 8 GiB (an upper bound of what enqueue_triangle takes)
-    const size_t per_block = sizeof(unsigned) * (size_t)std::max(1LL, G.max_bitmap_words);
-    nd.scratch = per_block * std::max<size_t>(1, std::min<size_t>((size_t)sm_count() * 3, ((size_t)8 << 30) / per_block));
-  }
+  if (!clique && triangle_by_tables(G)) nd.scratch = triangle_scratch(G);
   return nd;
 }
 }  // namespace
