@@ -267,6 +267,29 @@ DevGraph* find_graph(fsgc_ctx* c, int gid) {
   return it == c->graphs.end() ? nullptr : it->second;
 }
 
+// Captured pattern-set launches of graph `gid` (all graphs when gid < 0); its
+// sets start over with a direct call, which builds what the graph lacks.
+void drop_set_graphs(fsgc_ctx* c, int gid) {
+  for (auto it = c->set_graphs.begin(); it != c->set_graphs.end();) {
+    if (gid < 0 || it->second.gid == gid) {
+      cudaGraphExecDestroy(it->second.exec);
+      it = c->set_graphs.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  for (auto it = c->set_seen.begin(); it != c->set_seen.end();) {
+    if (gid < 0 || memcmp(it->first.data(), &gid, sizeof(gid)) == 0) it = c->set_seen.erase(it);
+    else ++it;
+  }
+}
+
+// Lets structures of the graph that once found no room be tried again when there
+// is more of it; captured sets start over then.
+void look_for_room(fsgc_ctx* c, int gid, DevGraph* g) {
+  if (fsgc::room_again(*g)) drop_set_graphs(c, gid);
+}
+
 // Host checks of a batch and the divisors of its patterns (context lock held).
 int plan_tasks(fsgc_ctx* c, const fsgc_task* tasks, int nt, std::vector<u64>& aut) {
   aut.assign((size_t)nt, 1);
@@ -276,6 +299,7 @@ int plan_tasks(fsgc_ctx* c, const fsgc_task* tasks, int nt, std::vector<u64>& au
     DevGraph* g = find_graph(c, tasks[t].gid);
     if (!g) return fail(c, FSGC_ENOTFOUND, "task %d: unknown graph %d", t, tasks[t].gid);
     if (g->ngraphs > 0) return fail(c, FSGC_EINVAL, "task %d: graph %d is packed; use fsgc_count_packed", t, tasks[t].gid);
+    look_for_room(c, tasks[t].gid, g);
     if (mo.nodes >= 3 && !pattern_too_large(mo, *g)) {
       const int st = automorphisms(c, mo, &aut[(size_t)t], c->exact_placements);
       if (st != FSGC_OK) return st;
@@ -353,23 +377,6 @@ int count_tasks(fsgc_ctx* c, const fsgc_task* tasks, int nt, fsgc_result* res) {
   if (st != FSGC_OK) return fail(c, st, "a counting kernel gave up a bounded wait; the counts are void");
   for (int t = 0; t < nt; t++) finish_task(t, jobs, aut, c->h_slots, c->events.data(), res);
   return FSGC_OK;
-}
-
-// Captured pattern-set launches of graph `gid` (all graphs when gid < 0); its
-// sets start over with a direct call, which builds what the graph lacks.
-void drop_set_graphs(fsgc_ctx* c, int gid) {
-  for (auto it = c->set_graphs.begin(); it != c->set_graphs.end();) {
-    if (gid < 0 || it->second.gid == gid) {
-      cudaGraphExecDestroy(it->second.exec);
-      it = c->set_graphs.erase(it);
-    } else {
-      ++it;
-    }
-  }
-  for (auto it = c->set_seen.begin(); it != c->set_seen.end();) {
-    if (gid < 0 || memcmp(it->first.data(), &gid, sizeof(gid)) == 0) it = c->set_seen.erase(it);
-    else ++it;
-  }
 }
 
 }  // namespace
@@ -739,6 +746,7 @@ int fsgc_count_packed(fsgc_ctx* c, int gid, const fsgc_matching_order* mo, fsgc_
   if (!g) return fail(c, FSGC_ENOTFOUND, "unknown graph %d", gid);
   if (g->ngraphs == 0) return fail(c, FSGC_EINVAL, "graph %d is not packed", gid);
   if (!mo_valid(*mo)) return fail(c, FSGC_EINVAL, "malformed matching order");
+  look_for_room(c, gid, g);
   const int ng = g->ngraphs;
   // pattern size (vertices, directed entries) for the per-member early return
   long long pn = mo->nodes, pm = 0;
@@ -826,6 +834,7 @@ int fsgc_graph_prepare_all(fsgc_ctx* c, int gid) {
   cudaSetDevice(c->device);
   DevGraph* g = find_graph(c, gid);
   if (!g) return fail(c, FSGC_ENOTFOUND, "unknown graph %d", gid);
+  look_for_room(c, gid, g);
   const int st = fsgc::prepare_all(*g, c->stream, &c->launches, c->work);
   if (st != FSGC_OK) return fail(c, st, "graph preparation failed: %s", cudaGetErrorString(cudaGetLastError()));
   return FSGC_OK;
@@ -875,6 +884,7 @@ int fsgc_count_exact(fsgc_ctx* c, int gid, const fsgc_matching_order* mo, fsgc_e
   DevGraph* g = find_graph(c, gid);
   if (!g) return fail(c, FSGC_ENOTFOUND, "unknown graph %d", gid);
   if (g->ngraphs > 0) return fail(c, FSGC_EUNSUPPORTED, "exact counts of packed graphs are not supported");
+  look_for_room(c, gid, g);
   if (pattern_too_large(*mo, *g)) {
     out->flags = FSGC_FLAG_PATTERN_TOO_LARGE;
     out->core_type = (mo->nodes == 3) ? ((__builtin_popcount(mo->list[1]) == 1) ? FSGC_CORE_WEDGE : FSGC_CORE_TRIANGLE)

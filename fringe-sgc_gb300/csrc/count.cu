@@ -1457,6 +1457,7 @@ int ensure_bit_matrix(DevGraph& G, cudaStream_t s, uint64_t* launches) {
     cudaGetLastError();
     G.bits = nullptr;
     G.bits_failed = true;
+    note_no_room(G, bytes);
     return FSGC_EUNSUPPORTED;
   }
   cudaMemsetAsync(G.bits, 0, bytes, s);
@@ -1817,6 +1818,26 @@ int check_tuning(const fsgc_tuning& t) {
                   t.triangle_stage_max % 32 == 0 && t.general_lane_venn_max >= 0 &&
                   t.general_lane_venn_max <= (1 << 20) && t.general_blocks_per_sm >= 1 && t.general_blocks_per_sm <= 16;
   return ok ? FSGC_OK : FSGC_EINVAL;
+}
+
+void note_no_room(DevGraph& G, size_t need) {
+  size_t free_now = 0, total = 0;
+  if (cudaMemGetInfo(&free_now, &total) != cudaSuccess) cudaGetLastError();
+  // more than was free, by a page, and enough for it
+  G.room_from = std::max(std::max(need, free_now + ((size_t)2 << 20)), G.room_from);
+}
+
+bool room_again(DevGraph& G) {
+  if (!G.rank_failed && !G.bits_failed) return false;
+  size_t free_now = 0, total = 0;
+  if (cudaMemGetInfo(&free_now, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (free_now < G.room_from) return false;
+  G.rank_failed = G.bits_failed = false;
+  G.room_from = 0;
+  return true;
 }
 
 size_t fast_structure_bytes(const DevGraph& G) { return G.rank_bytes + (G.bits ? bit_matrix_bytes(G) : 0); }

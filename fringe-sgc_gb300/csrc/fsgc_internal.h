@@ -69,9 +69,10 @@ struct DevGraph {
   int* rtab = nullptr;  // boundary table of the first rrows lists, rK columns
   int rrows = 0, rK = 0;
   size_t rank_bytes = 0;     // of the copy (0: there is none)
-  bool rank_failed = false;  // no room for the copy: not tried again
+  bool rank_failed = false;  // no room for the copy: not tried again before room_again()
   unsigned* bits = nullptr;  // lazily: adjacency bit matrix of a small graph (general cores)
-  bool bits_failed = false;  // no room for it: not tried again
+  bool bits_failed = false;  // no room for it, likewise
+  size_t room_from = 0;      // free device bytes at which what failed is tried again
   bool lean = false;  // neither of the two is built: counts take the paths without them
   // the reference's degree-relabel gate for the triangle core
   // (src/fringeCount.cu:1237, 1342-1344): vertex roles follow (deg, id) order
@@ -239,6 +240,11 @@ int prepare_all(DevGraph& g, cudaStream_t s, uint64_t* launches, DevWork& work);
 // is in flight).
 size_t fast_structure_bytes(const DevGraph& g);
 void free_fast_structures(DevGraph& g);
+// Notes that a structure which takes `need` bytes to build found no room.
+void note_no_room(DevGraph& g, size_t need);
+// Whether structures that found no room may be tried again, which the caller then
+// lets happen on the context's stream; false as long as no more is free than then.
+bool room_again(DevGraph& g);
 // Scratch-arena bytes a count of `mo` on the prepared graph `g` grows to.
 size_t count_scratch_bytes(const fsgc_matching_order& mo, const DevGraph& g, const fsgc_tuning& t);
 // FSGC_EINVAL unless every field of `t` is in its documented range.

@@ -1296,7 +1296,6 @@ int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& 
       G.roff = G.radj = G.rdeg = G.oid = G.rrev = G.rtab = nullptr;
       G.rrows = G.rK = 0;
       cudaGetLastError();
-      if (st == FSGC_EUNSUPPORTED) G.rank_failed = true;
     }
     return st;
   };
@@ -1320,7 +1319,11 @@ int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& 
       !get((void**)&G.radj, sizeof(int) * (size_t)m) || !get((void**)&G.rrev, sizeof(int) * (size_t)m) ||
       !get((void**)&G.radj16, sizeof(short) * ((size_t)m + 8))) {
     cudaStreamSynchronize(s);
-    return drop(FSGC_EUNSUPPORTED);  // no room: the count takes the path without this copy
+    drop(FSGC_EUNSUPPORTED);  // no room: the count takes the path without this copy
+    cudaStreamSynchronize(s);  // what was had is free again
+    G.rank_failed = true;
+    note_no_room(G, 3 * sizeof(int) * big + tb + sizeof(int) * ((size_t)4 * n + 64) + (2 * sizeof(int) + sizeof(short)) * (size_t)m);
+    return FSGC_EUNSUPPORTED;
   }
   const int vg = grid_for((long long)n + 1, kTPB, 16);
   // every pass indexes with what the sort or scan before it wrote
