@@ -1803,7 +1803,7 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
   }
   const bool clique = (f[IUVW] == 1) && (f[IUV] + f[IUW] + f[IVW] == 0) &&
                       ((f[IU] == 0) + (f[IV] == 0) + (f[IW] == 0) >= 2);
-  if (!clique && triangle_by_tables(G)) nd.scratch = triangle_scratch(G);
+  if (!clique && triangle_by_tables(G, clique)) nd.scratch = triangle_scratch(G);
   return nd;
 }
 }  // namespace
@@ -2077,7 +2077,7 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
     tp.relabel = G.tri_relabel ? 1 : 0;
     rotations3(f, false, tp.rot);
     if (me == 0) return FSGC_OK;
-    if (triangle_by_tables(G))
+    if (triangle_by_tables(G, clique))
       return enqueue_triangle(G, gv, tp, std::is_same<A, X128>::value, job.d_slot, s, launches, work);
     triangle_core_kernel<A><<<grid_for(me, TPB, 8), TPB, 0, s>>>(gv, tp, job.d_slot);
     *launches += 1;

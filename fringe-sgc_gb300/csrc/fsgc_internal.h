@@ -182,7 +182,7 @@ constexpr int kTriNarrowK = 256, kTriNarrowRows = 6400, kTriNarrowLists = 4096;
 __host__ __device__ inline bool triangle_wide(int k, int lists) {
   return k > kTriNarrowK || lists > kTriNarrowLists || (long long)k * (((lists + 31) >> 5) | 1) > kTriNarrowRows;
 }
-bool triangle_by_tables(const DevGraph& G);  // out-degrees small enough for that path
+bool triangle_by_tables(const DevGraph& G, bool clique);  // out-degrees for which that path is taken
 size_t triangle_scratch(const DevGraph& G);  // work-arena bytes of its modes other than the 4-cliques
 int enqueue_triangle(DevGraph& G, const GView& gv, const TrianglePattern& tp, bool exact, u64* slot, cudaStream_t s,
                      uint64_t* launches, DevWork& work);
