@@ -1499,6 +1499,18 @@ bool bit_sets_for(const GenParams& p, bool exact, int n, BitSets& bs) {
   return true;
 }
 
+// Parts that a list entry's third vertices are split into: enough tasks for the
+// warps to end together, but fewer than the longest list has entries and than four
+// times those of the lists that entries lie in on average, where most parts are
+// empty.  Split 32 ways whatever the lists, a path of 4,096 took 0.20 ms (searching
+// lists 0.03 ms, now 0.03 ms), a square grid 0.27 ms (0.21, now 0.12).
+int bits_parts(const DevGraph& G, long long warps) {
+  const double most = std::min((double)G.maxdeg, 4 * G.mean_end_degree);
+  int parts = 1;
+  while (parts < 32 && 2 * parts < most && G.m * parts < warps * 32) parts *= 2;
+  return parts;
+}
+
 template <int D, class A>
 int launch_bits(const GView& gv, const GenParams& gp, BitSets bs, const unsigned* mat, unsigned long long* queue, u64* slot,
                 int blocks, cudaStream_t s) {
@@ -2125,9 +2137,7 @@ int enqueue_count_a(CountJob& job, cudaStream_t s, uint64_t* launches, DevWork& 
   if (bit_sets_for(*gp, gp->exact || !std::is_same<A, u64>::value, G.n, bs)) {
     st = ensure_bit_matrix(G, s, launches);
     if (st == FSGC_OK) {
-      // enough tasks for the warps to end together
-      bs.parts = 1;
-      while (bs.parts < 32 && G.m * bs.parts < (long long)blocks * kGenWarps * 32) bs.parts *= 2;
+      bs.parts = bits_parts(G, (long long)blocks * kGenWarps);
       if (ns <= 32) st = launch_bits<32, A>(gv, *gp, bs, G.bits, queue, job.d_slot, blocks, s);
       else if (ns <= 64) st = launch_bits<64, A>(gv, *gp, bs, G.bits, queue, job.d_slot, blocks, s);
       else st = launch_bits<128, A>(gv, *gp, bs, G.bits, queue, job.d_slot, blocks, s);

@@ -52,6 +52,7 @@ struct DevGraph {
   int* wide = nullptr;             // vertices whose triangles take a wide block each (triangle_wide)
   int nwide = 0;
   long long max_bitmap_words = 0;  // max over v of outdeg(v) * ceil(deg(v) / 32)
+  double mean_end_degree = 0;      // over the list entries: mean degree of their vertices
   u64* vtri2 = nullptr;  // lazily
   unsigned* esup = nullptr;  // lazily: per list entry (u, v), |N(u) & N(v)|
   // wedge core: offsets of chunk boundaries in the lists of high-degree vertices (lazily)

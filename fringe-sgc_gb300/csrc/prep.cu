@@ -540,27 +540,31 @@ __global__ void supports_back_kernel(int me, const int* __restrict__ place, cons
 }
 
 // Largest out-degree, largest out-degree * ceil(deg / 32) (bitmap rows), the
-// number of vertices whose triangles take a wide block, and the sum of squares.
+// number of vertices whose triangles take a wide block, and the sums of squares of
+// out-degrees and (stats[5]) of degrees.
 __global__ void outdeg_stats_kernel(GView g, unsigned long long* __restrict__ stats) {
-  unsigned long long k1 = 0, k2 = 0, wide = 0, squares = 0;
+  unsigned long long k1 = 0, k2 = 0, wide = 0, squares = 0, ends = 0;
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += gridDim.x * blockDim.x) {
     const unsigned long long k = (unsigned long long)(g.ooff[v + 1] - g.ooff[v]);
     k1 = max(k1, k);
     k2 = max(k2, k * (unsigned long long)((g.deg[v] + 31) >> 5));
     wide += k >= 2 && triangle_wide((int)k, g.deg[v]);
     squares += k * k;
+    ends += (unsigned long long)g.deg[v] * (unsigned long long)g.deg[v];
   }
   for (int o = 16; o > 0; o >>= 1) {
     k1 = max(k1, __shfl_down_sync(0xffffffffu, k1, o));
     k2 = max(k2, __shfl_down_sync(0xffffffffu, k2, o));
     wide += __shfl_down_sync(0xffffffffu, wide, o);
     squares += __shfl_down_sync(0xffffffffu, squares, o);
+    ends += __shfl_down_sync(0xffffffffu, ends, o);
   }
   if ((threadIdx.x & 31) == 0) {
     atomicMax(stats, k1);
     atomicMax(stats + 1, k2);
     if (wide) atomicAdd(stats + 2, wide);
     if (squares) atomicAdd(stats + 4, squares);
+    if (ends) atomicAdd(stats + 5, ends);
   }
 }
 
@@ -743,7 +747,8 @@ int prepare_graph(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_u64) {
   orient_fill_kernel<<<wgrid, kTPB, 0, s>>>(v, g.oadj, g.osrc);
   *launches += 5;
   u64* d_stats = d_u64 + 2;
-  FSGC_TRY(cudaMemsetAsync(d_stats, 0, 5 * sizeof(u64), s));  // the last two: the list's fill count, sum of squares
+  // after the first three: the list's fill count, sums of squares of out-degrees and degrees
+  FSGC_TRY(cudaMemsetAsync(d_stats, 0, 6 * sizeof(u64), s));
   outdeg_stats_kernel<<<grid_for(n, kTPB, 8), kTPB, 0, s>>>(v, d_stats);
   *launches += 1;
   // supports and triangle total
@@ -761,8 +766,8 @@ int prepare_graph(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_u64) {
     triangle_support_kernel<<<grid_for(me, kTPB, 8), kTPB, 0, s>>>(v, g.osup, d_tri);
     *launches += 1;
   }
-  u64 stats[4] = {0, 0, 0, 0};
-  FSGC_TRY(cudaMemcpyAsync(stats, d_tri, 4 * sizeof(u64), cudaMemcpyDeviceToHost, s));
+  u64 stats[7] = {0};
+  FSGC_TRY(cudaMemcpyAsync(stats, d_tri, sizeof(stats), cudaMemcpyDeviceToHost, s));
   FSGC_TRY(cudaFreeAsync(odeg, s));
   FSGC_TRY(cudaFreeAsync(tiles, s));
   FSGC_TRY(cudaStreamSynchronize(s));
@@ -770,6 +775,7 @@ int prepare_graph(DevGraph& g, cudaStream_t s, uint64_t* launches, u64* d_u64) {
   g.triangles = (long long)stats[0];
   g.max_outdeg = (long long)stats[1];
   g.max_bitmap_words = (long long)stats[2];
+  g.mean_end_degree = g.m > 0 ? (double)stats[6] / (double)g.m : 0;
   if (stats[3] > 0) {
     FSGC_TRY(cudaMallocAsync((void**)&g.wide, sizeof(int) * (size_t)stats[3], s));
     wide_list_kernel<<<grid_for(n, kTPB, 8), kTPB, 0, s>>>(v, g.wide, reinterpret_cast<int*>(d_stats + 3));
