@@ -127,12 +127,20 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
   const bool same = f_v == f_w;
   A total = A(0);
   auto span = [&](const int* nb, int d, int first, int stride, A& p_sum, A& q_sum, A& acc) {
-    for (int t = first; t < d; t += stride) {
-      const int dx = g.deg[__ldg(nb + t)] - 1;
-      const A p = nck_a<A>(dx, f_v), q = same ? p : nck_a<A>(dx, f_w);
-      acc += same ? p * p_sum : p * q_sum + q * p_sum;
-      p_sum += p;
-      q_sum += q;
+    for (int t0 = first; t0 < d; t0 += 4 * stride) {
+      int x[4], dx[4];  // four entries and their degrees in flight
+#pragma unroll
+      for (int k = 0; k < 4; k++) x[k] = d - t0 > k * stride ? __ldg(nb + t0 + k * stride) : -1;
+#pragma unroll
+      for (int k = 0; k < 4; k++) dx[k] = x[k] >= 0 ? __ldg(g.deg + x[k]) - 1 : 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (x[k] < 0) break;
+        const A p = nck_a<A>(dx[k], f_v), q = same ? p : nck_a<A>(dx[k], f_w);
+        acc += same ? p * p_sum : p * q_sum + q * p_sum;
+        p_sum += p;
+        q_sum += q;
+      }
     }
   };
   // consecutive vertices go to different blocks: hubs are often neighbours by id
@@ -1096,21 +1104,37 @@ __global__ void rank_assign_kernel(GView g, const int* __restrict__ oid, int* __
   }
 }
 
+// Calls f(r, first, step) for every rank r whose list the thread takes part in, from
+// entry `first` on, every `step`-th: the whole grid for the leading ranks with long
+// lists (all hubs of an ordinary graph), a warp for every other.  A warp alone took
+// 40 ms for the two passes over a list of a million entries, 12 ns an entry and pass.
+// The grid's turns take 1 to 2 us each, so rank r has one as long as its list takes
+// a warp longer than the r turns before it: two hubs of 30,000 are two turns, a graph
+// of lists of 9,000 has forty.
+constexpr int kGridList = 4096, kGridTurn = 120;
+template <class F>
+__device__ __forceinline__ void each_list(const int* __restrict__ rdeg, int n, F f) {
+  const int at = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+  int long_lists = 0;
+  for (; long_lists < n && rdeg[long_lists] > kGridList + (long long)kGridTurn * long_lists; long_lists++)
+    f(long_lists, at, all);
+  for (int r = long_lists + (at >> 5); r < n; r += all >> 5) f(r, at & 31, 32);
+}
+
 // (neighbour's rank, own rank) per list entry, owners in rank order: a stable
 // sort by the first gives every vertex its neighbours' ranks in ascending
 // order, because a symmetric graph is its own transpose.
 __global__ void rank_entries_kernel(GView g, const int* __restrict__ oid, const int* __restrict__ rank,
-                                    const int* __restrict__ roff, unsigned* __restrict__ key, int* __restrict__ val) {
-  const int lane = threadIdx.x & 31;
-  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (int r = wid; r < g.n; r += nw) {
-    const int v = oid[r], o = roff[r], d = g.deg[v];
-    const int* nb = g.adj + g.off[v];
-    for (int t = lane; t < d; t += 32) {
+                                    const int* __restrict__ roff, const int* __restrict__ rdeg,
+                                    unsigned* __restrict__ key, int* __restrict__ val) {
+  each_list(rdeg, g.n, [&](int r, int first, int step) {
+    const int o = roff[r], d = rdeg[r];
+    const int* nb = g.adj + g.off[oid[r]];
+    for (int t = first; t < d; t += step) {
       key[o + t] = (unsigned)rank[__ldg(nb + t)];
       val[o + t] = r;
     }
-  }
+  });
 }
 
 // ranks with degree >= 2^(k + 4), k = 0..15 (degrees descend)
@@ -1143,11 +1167,9 @@ __global__ void rank_low16_kernel(const int* __restrict__ radj, int m, unsigned 
 // entries of N(u) up to and including v, per list entry (v, u)
 __global__ void rank_reverse_kernel(const int* __restrict__ roff, const int* __restrict__ radj, const int* __restrict__ rdeg,
                                     int n, const int* __restrict__ tab, int rows, int K, int* __restrict__ rev) {
-  const int lane = threadIdx.x & 31;
-  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (int v = wid; v < n; v += nw) {
+  each_list(rdeg, n, [&](int v, int first, int step) {
     const int vb = roff[v], d = rdeg[v];
-    for (int t = lane; t < d; t += 32) {
+    for (int t = first; t < d; t += step) {
       const int u = __ldg(radj + vb + t), ub = roff[u], du = rdeg[u];
       int lo = 0, hi = du;
       if (u < rows) {  // the boundary table narrows the search
@@ -1162,7 +1184,7 @@ __global__ void rank_reverse_kernel(const int* __restrict__ roff, const int* __r
       }
       rev[vb + t] = lo;
     }
-  }
+  });
 }
 
 int bits_for(unsigned x) {
@@ -1344,7 +1366,7 @@ int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& 
   rank_assign_kernel<<<vg, kTPB, 0, s>>>(gv, G.oid, rank, G.rdeg);
   size_t tt = tb;
   if (cub::DeviceScan::ExclusiveSum(temp, tt, G.rdeg, G.roff, n + 1, s) != cudaSuccess) return drop(FSGC_ECUDA);
-  rank_entries_kernel<<<grid_for((long long)n * 32, kTPB, 16), kTPB, 0, s>>>(gv, G.oid, rank, G.roff, k1, v1);
+  rank_entries_kernel<<<grid_for((long long)n * 32, kTPB, 16), kTPB, 0, s>>>(gv, G.oid, rank, G.roff, G.rdeg, k1, v1);
   if (!sort(G.radj, m, rank_bits)) return drop(FSGC_ECUDA);
   *launches += 2;
   // boundary table of the long lists (ordinary graphs; a packed graph's members
