@@ -1774,6 +1774,7 @@ int ensure_plain_scratch(Scratch& sc, size_t need, cudaStream_t s) {
 namespace {
 struct Needs {
   bool chunk_table = false;  // wedge core with a fringe-free centre
+  bool pairs = false;        // which evaluates its pairs one by one in rank order
   bool vertex_triangles = false;
   bool entry_supports = false;  // general wedge core
   bool bit_matrix = false;      // general cores and that one, on a small graph
@@ -1803,6 +1804,7 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
     }
     if (f[IUVW] == 0 && f[IUV] == 0 && f[IUW] == 0 && f[IU] == 0) {
       nd.chunk_table = true;
+      nd.pairs = wedge_pass(G, WedgeParams{f[IV], f[IVW], f[IW], 0, 0}) == kPairsPass;
       if (G.maxdeg > std::min(kWDvMax, std::max(16, t.wedge_small_max_degree))) {
         const long long gs = G.maxdeg;
         nd.scratch = (size_t)sm_count() * ((size_t)2 * gs * sizeof(long long) + (size_t)(gs + 1) * sizeof(int));
@@ -1868,7 +1870,7 @@ int prepare_for_count(const fsgc_matching_order& mo, DevGraph& G, cudaStream_t s
   if (st != FSGC_OK) return st;
   const Needs nd = needs_of(mo, G, work.tune);
   if (nd.chunk_table) {
-    st = ensure_rank_order(G, s, launches, work);
+    st = nd.pairs && pairs_by_chunks(G, 1) ? FSGC_EUNSUPPORTED : ensure_rank_order(G, s, launches, work);
     if (st == FSGC_EUNSUPPORTED) st = ensure_chunk_table(G, s, launches, work.small + 9);
     if (st != FSGC_OK) return st;
   }
@@ -1887,13 +1889,13 @@ int prepare_for_count(const fsgc_matching_order& mo, DevGraph& G, cudaStream_t s
   return cudaStreamSynchronize(s) == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
 }
 
-// The chunk table is for graphs without a copy in rank order: beside one, only
-// exact counts beyond its bound read it, and they build it.
+// The chunk table is for graphs without a copy in rank order and dense ones: beside
+// a copy, only exact counts beyond its bound read it elsewhere, and they build it.
 int prepare_all(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) {
   int st = prepare_graph(G, s, launches, work.small);
   if (st == FSGC_OK) {
     st = ensure_rank_order(G, s, launches, work);
-    if (st == FSGC_EUNSUPPORTED)  // counted another way
+    if (st == FSGC_EUNSUPPORTED || (st == FSGC_OK && pairs_by_chunks(G, 1)))
       st = G.ngraphs == 0 ? ensure_chunk_table(G, s, launches, work.small + 9) : FSGC_OK;
   }
   if (st == FSGC_OK) st = ensure_vertex_triangles(G, s, launches);
@@ -1907,20 +1909,15 @@ int prepare_all(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) 
 }
 
 namespace {
-// The fringe-free-centre wedge core for a set of patterns: in rank order where
-// the graph takes that path, else by both pair kernels: endpoints of degree <= kWDvMax, then hub endpoints (cursors and
-// segment offsets in the work arena).
+// The fringe-free-centre wedge core for a set of patterns by both pair kernels:
+// endpoints of degree <= kWDvMax, then hub endpoints (cursors and segment offsets in
+// the work arena).
 template <int NP, class A>
-int launch_wedge_set(DevGraph& G, const GView& gv, const WedgeSet& ws0, cudaStream_t s, uint64_t* launches,
-                     DevWork& work) {
-  const size_t arena = wedge_rank_scratch(G);
-  int st = wedge_rank_size_ok(G) && arena > 0 ? ensure_plain_scratch(work.tri, std::max(arena, work.tri.bytes), s) : FSGC_OK;
-  if (st != FSGC_OK) return st;
-  st = enqueue_wedge_rank(G, gv, ws0.w, ws0.slot, ws0.np, std::is_same<A, X128>::value, s, launches, work);
-  if (st != FSGC_EUNSUPPORTED) return st;
+int launch_wedge_chunks(DevGraph& G, const GView& gv, const WedgeSet& ws0, cudaStream_t s, uint64_t* launches,
+                        DevWork& work) {
   int* q1 = reinterpret_cast<int*>(work.small + 7);
   int* q2 = reinterpret_cast<int*>(work.small + 8);
-  st = ensure_chunk_table(G, s, launches, work.small + 9);
+  int st = ensure_chunk_table(G, s, launches, work.small + 9);
   if (st != FSGC_OK) return st;
   const ChunkTable tab{G.ctab_id, G.ctab_pos, G.ctab_K};
   cudaMemsetAsync(q1, 0, 2 * sizeof(u64), s);
@@ -1947,6 +1944,34 @@ int launch_wedge_set(DevGraph& G, const GView& gv, const WedgeSet& ws0, cudaStre
     *launches += 1;
   }
   return cudaGetLastError() == cudaSuccess ? FSGC_OK : FSGC_ECUDA;
+}
+
+// The fringe-free-centre wedge core for a set of patterns: in rank order where the
+// graph takes that path, but patterns whose pairs are evaluated one by one by chunks
+// where that is the better path for as many of them.
+template <int NP, class A>
+int launch_wedge_set(DevGraph& G, const GView& gv, const WedgeSet& ws, cudaStream_t s, uint64_t* launches, DevWork& work) {
+  const bool none = !wedge_rank_size_ok(G) || (!G.radj && (G.lean || G.rank_failed));  // no copy, nor will there be
+  if (none) return launch_wedge_chunks<NP, A>(G, gv, ws, s, launches, work);
+  int evaluated = 0;
+  if (std::is_same<A, u64>::value)
+    for (int i = 0; i < ws.np; i++) evaluated += wedge_pass(G, ws.w[i]) == kPairsPass;
+  const int from = !pairs_by_chunks(G, evaluated) ? kPairsPass + 1 : sums_join_pairs(G) ? kSumsPass : kPairsPass;
+  WedgeSet rank = ws, pairs = ws;
+  rank.np = pairs.np = 0;
+  for (int i = 0; i < ws.np; i++) {
+    WedgeSet& to = wedge_pass(G, ws.w[i]) >= from ? pairs : rank;
+    to.w[to.np] = ws.w[i];
+    to.slot[to.np++] = ws.slot[i];
+  }
+  int st = FSGC_OK;
+  if (pairs.np > 0) st = launch_wedge_chunks<NP, A>(G, gv, pairs, s, launches, work);
+  if (st != FSGC_OK || rank.np == 0) return st;
+  const size_t arena = wedge_rank_scratch(G);
+  if (arena > 0) st = ensure_plain_scratch(work.tri, std::max(arena, work.tri.bytes), s);
+  if (st != FSGC_OK) return st;
+  st = enqueue_wedge_rank(G, gv, rank.w, rank.slot, rank.np, std::is_same<A, X128>::value, s, launches, work);
+  return st == FSGC_EUNSUPPORTED ? launch_wedge_chunks<NP, A>(G, gv, rank, s, launches, work) : st;
 }
 
 template <class A>

@@ -1226,6 +1226,11 @@ PairForm pair_form(const WedgeParams& p, bool exact) {
   return f;
 }
 
+// Binomials of the pattern's sums, the sums with C common neighbours among them.
+bool pattern_fits(const DevGraph& G, const WedgeParams& p) {
+  return binomials_fit(G.maxdeg, std::max(p.f_v, std::max(p.f_vw, p.f_w)));
+}
+
 // Whether the pattern's residual is a multiple of C (C - 1) alone.
 bool counts_four_cycles(const WedgeParams& p, long long* mult) {
   if (p.f_v == 1 && p.f_w == 1 && p.f_vw == 0) *mult = -4;       // C ((dx-1)(dy-1) - (C-1))
@@ -1276,7 +1281,7 @@ int enqueue_rank_a(DevGraph& G, const GView& gv, const WedgeParams* pats, u64* c
       ord.np = 0;
       continue;
     }
-    const bool fits = std::is_same<A, u128>::value || binomials_fit(G.maxdeg, std::max(p.f_v, std::max(p.f_vw, p.f_w)));
+    const bool fits = std::is_same<A, u128>::value || pattern_fits(G, p);
     // no shared fringe and none on one end: W does not depend on C, as long as
     // no binomial wraps before its division
     if (fits && p.f_vw == 0 && std::min(p.f_v, p.f_w) == 0) continue;
@@ -1299,6 +1304,38 @@ int enqueue_rank_a(DevGraph& G, const GView& gv, const WedgeParams* pats, u64* c
 bool binomials_fit(int maxdeg, int k) {
   return k <= 2 || k * std::log2((double)std::max(2, maxdeg)) - std::lgamma((double)k) / std::log(2.0) < 63.0;
 }
+
+WedgePass wedge_pass(const DevGraph& G, const WedgeParams& p) {
+  long long mult = 0;
+  const bool fits = pattern_fits(G, p);
+  if (counts_four_cycles(p, &mult) || (fits && p.f_vw == 0 && std::min(p.f_v, p.f_w) == 0)) return kNoPass;
+  return pair_form(p, fits).kind == kGeneral ? kPairsPass : kSumsPass;
+}
+
+static double wedges_per_pair(const DevGraph& G) { return (double)G.m * G.mean_end_degree / ((double)G.n * (double)G.n); }
+
+// A pair costs the residual two evaluations and the chunk kernel one, which counts up
+// to four patterns in one pass: the better where most vertices are pairs with common
+// neighbours and none is a large hub.  With R wedges a pair of ids and S the mean
+// degree of an entry's vertex over the mean degree (ms, two and two fringes; three and
+// three; a set of three such and one other; by chunks and in rank order):
+//   uniform, n = 3,000, R = 0.09: 0.20 0.12; 0.22 0.16; 0.40 0.48
+//   n = 16,000, R = 0.16: 1.38 1.20; 1.70 1.87; 4.4 5.7   n = 8,000, R = 0.32: 0.70 0.71; 0.86 1.15; 2.1 3.4
+//   n = 5,000, R = 8: 0.84 0.97; 1.22 1.71; 2.7 4.8       n = 5,000, R = 0.055: 0.30 0.13; 0.34 0.16; 0.62 0.53
+//   RMAT n = 1,024, R = 2, S = 4.7: 0.10 0.14; 0.13 0.22; 0.31 0.62
+//   RMAT n = 4,096, R = 1.1, S = 8: 0.31 0.28; 0.42 0.44; 1.10 1.31
+//   RMAT n = 16,384, R = 0.6, S = 14: 1.4 1.1; 1.9 1.6; 5.8 5.0
+//   cliques of 600 and 1,200, R = n - 1: 0.39 0.26, 2.3 1.1; 0.40 0.29, 2.3 1.2; 0.47 1.03, 2.5 4.5
+bool pairs_by_chunks(const DevGraph& G, int count) {
+  if (count == 0 || G.ngraphs > 0 || G.m == 0) return false;
+  const double R = wedges_per_pair(G), S = G.mean_end_degree * (double)G.n / (double)G.m;
+  return count == 1 ? R >= 0.25 && R <= 256 && S <= 6.5 : R >= 0.08 && S <= 9;
+}
+
+// From about 16 wedges a pair of ids (the set above, its fourth pattern in rank order and
+// by chunks): cliques of 600 0.68 0.47, of 200 0.16 0.12; uniform R = 67 0.30 0.27,
+// R = 27 0.66 0.64, R = 8 2.5 2.7.
+bool sums_join_pairs(const DevGraph& G) { return wedges_per_pair(G) >= 16; }
 
 int ensure_rank_order(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) {
   if (G.radj) return FSGC_OK;
