@@ -8,8 +8,8 @@ per context, and this module picks them per graph by timing:
                           runs in the shared-memory counter kernel (higher
                           degrees go to the hub kernel) on graphs that do not
                           take the rank-order path
-  triangle_walk_ratio,    kept for saved settings; no kernel reads them, so
-  triangle_stage_max      the default wins unless timing noise says otherwise
+  triangle_walk_ratio,    kept for saved settings; no kernel reads them, and the
+  triangle_stage_max      command below leaves them at their defaults
   general_lane_venn_max   general cores: Venn rows up to this many list
                           entries are built by one lane, longer ones by a warp
   general_blocks_per_sm   general cores: the task granularity of the grid
@@ -38,6 +38,8 @@ CANDIDATES = {
     "general_lane_venn_max": [0, 32, 96, 256, 1 << 20],
     "general_blocks_per_sm": [2, 4, 8, 12],
 }
+# fields that no kernel reads
+UNREAD = {"triangle_walk_ratio", "triangle_stage_max"}
 # core types (fsgc_result.core_type) whose kernels each field steers
 STEERS = {
     "wedge_small_max_degree": {3},
@@ -131,7 +133,8 @@ def main():
     with fsgc.Context(0) as ctx:
         gid = ctx.upload(g)
         ctx.prepare(gid)
-        values, report = tune(ctx, gid, mos, args.repeats, log=lambda s: print(s, file=sys.stderr, flush=True))
+        fields = [f for f in CANDIDATES if f not in UNREAD]
+        values, report = tune(ctx, gid, mos, args.repeats, fields, log=lambda s: print(s, file=sys.stderr, flush=True))
         ctx.release(gid)
     key = graph_key(g.n, g.m, int(g.degrees().max()))
     save(args.out, key, values, report, note=f"RMAT scale {args.scale}, {len(mos)} patterns")
