@@ -240,16 +240,17 @@ def edges_per_second(m, per_pattern_ms):
 
 def measured_traffic(pattern, g):
     """DRAM bytes (read + write) of one count of `pattern` on this graph, from the
-    ncu capture recorded in profiles/dram_traffic.json (null when the capture
-    was of another pattern or graph size)."""
+    ncu captures recorded in profiles/dram_traffic.json (null when none is of this
+    pattern and graph size)."""
     p = os.path.join(ROOT, "profiles", "dram_traffic.json")
     if not os.path.exists(p):
         return None
     with open(p) as f:
         rec = json.load(f)
-    if rec.get("pattern") != pattern or rec.get("n") != g.n or rec.get("m") != g.m:
-        return None
-    return rec.get("dram_bytes")
+    for r in [rec] + rec.get("others", []):
+        if (r.get("pattern"), r.get("n"), r.get("m")) == (pattern, g.n, g.m):
+            return r.get("dram_bytes")
+    return None
 
 
 def max_over_ranks(values, world):

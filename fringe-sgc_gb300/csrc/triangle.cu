@@ -23,11 +23,13 @@
 // of the work arena.
 //
 // What bounds it: the lookups' instructions (a hash probe, five shuffles and a
-// share of a list load per entry, 21 of 32 lanes busy) and their latency; DRAM is
-// idle.  RMAT n = 600,011 (192M triangles), 4-clique with three fringes: rows by
-// binary searches in the arena 167 ms -> 55 ms; RMAT scale 16: 4-clique (one lane
-// per triangle, before) 129 -> 2.4 ms, with two tails 201 -> 2.7 ms, a mixed
-// triangle pattern (six rotations) 77 -> 17 ms, of which the placement sums
+// share of a list load per entry, 20 to 22 of 32 lanes busy) and their latency: on
+// RMAT n = 2^20 the schedulers issue in 43 (narrow blocks) and 38 of 100 cycles with
+// 36 % of the warps in flight, which wait for list reads and for shared memory; DRAM
+// runs at 1 % of its rate.  RMAT n = 600,011 (192M triangles), 4-clique with three
+// fringes: rows by binary searches in the arena 167 ms -> 57 ms; RMAT n = 65,536:
+// 4-clique (one lane per triangle, before) 129 -> 2.3 ms, with two tails 201 -> 2.6 ms,
+// a mixed triangle pattern (six rotations) 77 -> 18 ms, of which the placement sums
 // (fc3_ring instead of fc3) are half.
 #include <algorithm>
 #include <cstring>

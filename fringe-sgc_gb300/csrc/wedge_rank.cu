@@ -772,14 +772,15 @@ __device__ __noinline__ A scan_general(const RankView& r, const RankSet& rs, Ran
 // warp, through the residual formula as the words are read and cleared.  ORD:
 // the centres are restricted to u > v and every add returns the pairs it
 // closes, so there is nothing to evaluate.
-// What bounds it: instructions and list-read latency, not bytes or adds.  A
-// random shared-memory add costs 2.9 cycles per warp and SM, 10 ms for the
-// 3.5e10 wedges of RMAT scale 20; the walk (equal shares of padded segments,
-// three 8-byte loads a lane in flight) takes 44% of the time, the counter scan
-// 20%, the segments' ends 17%.  Whole counts on RMAT scale 20 (31M entries),
-// before -> after, with the two O(m) passes: one fringe on each end 344 -> 16 ms
-// (ORD), 4-cycle with opposite fringes 327 -> 80 ms, three fringes and one
-// 636 -> 95 ms.  The copy in rank order is built once per graph: 11 ms there.
+// What bounds it: instructions and list-read latency, not bytes or adds.  On RMAT
+// n = 2^20, 31M entries, the schedulers issue in 62 (ORD) and 64 of 100 cycles with
+// half the warps in flight, which wait for list reads (3.1 and 2.0 of a warp's cycles
+// an instruction), dependent instructions (2.1, 2.3) and barriers (1.8, 2.5); the
+// shared-memory adds, 2.9 cycles a warp and SM where they are random, are 13 and 12 %
+// of the time, DRAM 6 and 1.5 % of its rate.  Whole counts there, before -> after, with
+// the linear pass (1.4 to 2.4 ms) and the adjacent one (0.3 to 1.1 ms): one fringe on
+// each end 344 -> 17 ms (ORD), 4-cycle with opposite fringes 327 -> 87 ms, three
+// fringes and one 636 -> 98 ms.  The copy in rank order is built once per graph: 5 ms.
 template <bool ORD, class A>
 __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constant__ RankView r,
                                                             const __grid_constant__ RankSet rs,
