@@ -1804,7 +1804,7 @@ Needs needs_of(const fsgc_matching_order& mo, const DevGraph& G, const fsgc_tuni
     }
     if (f[IUVW] == 0 && f[IUV] == 0 && f[IUW] == 0 && f[IU] == 0) {
       nd.chunk_table = true;
-      nd.pairs = wedge_pass(G, WedgeParams{f[IV], f[IVW], f[IW], 0, 0}) == kPairsPass;
+      nd.pairs = wedge_pass(G, WedgeParams{f[IV], f[IVW], f[IW], 0, 0}, false) == kPairsPass;
       if (G.maxdeg > std::min(kWDvMax, std::max(16, t.wedge_small_max_degree))) {
         const long long gs = G.maxdeg;
         nd.scratch = (size_t)sm_count() * ((size_t)2 * gs * sizeof(long long) + (size_t)(gs + 1) * sizeof(int));
@@ -1870,7 +1870,7 @@ int prepare_for_count(const fsgc_matching_order& mo, DevGraph& G, cudaStream_t s
   if (st != FSGC_OK) return st;
   const Needs nd = needs_of(mo, G, work.tune);
   if (nd.chunk_table) {
-    st = nd.pairs && pairs_by_chunks(G, 1) ? FSGC_EUNSUPPORTED : ensure_rank_order(G, s, launches, work);
+    st = nd.pairs && pairs_by_chunks(G, 1, false) ? FSGC_EUNSUPPORTED : ensure_rank_order(G, s, launches, work);
     if (st == FSGC_EUNSUPPORTED) st = ensure_chunk_table(G, s, launches, work.small + 9);
     if (st != FSGC_OK) return st;
   }
@@ -1895,7 +1895,7 @@ int prepare_all(DevGraph& G, cudaStream_t s, uint64_t* launches, DevWork& work) 
   int st = prepare_graph(G, s, launches, work.small);
   if (st == FSGC_OK) {
     st = ensure_rank_order(G, s, launches, work);
-    if (st == FSGC_EUNSUPPORTED || (st == FSGC_OK && pairs_by_chunks(G, 1)))
+    if (st == FSGC_EUNSUPPORTED || (st == FSGC_OK && pairs_by_chunks(G, 1, false)))
       st = G.ngraphs == 0 ? ensure_chunk_table(G, s, launches, work.small + 9) : FSGC_OK;
   }
   if (st == FSGC_OK) st = ensure_vertex_triangles(G, s, launches);
@@ -1954,13 +1954,13 @@ int launch_wedge_set(DevGraph& G, const GView& gv, const WedgeSet& ws, cudaStrea
   const bool none = !wedge_rank_size_ok(G) || (!G.radj && (G.lean || G.rank_failed));  // no copy, nor will there be
   if (none) return launch_wedge_chunks<NP, A>(G, gv, ws, s, launches, work);
   int evaluated = 0;
-  if (std::is_same<A, u64>::value)
-    for (int i = 0; i < ws.np; i++) evaluated += wedge_pass(G, ws.w[i]) == kPairsPass;
-  const int from = !pairs_by_chunks(G, evaluated) ? kPairsPass + 1 : sums_join_pairs(G) ? kSumsPass : kPairsPass;
+  constexpr bool exact = std::is_same<A, X128>::value;
+  for (int i = 0; i < ws.np; i++) evaluated += wedge_pass(G, ws.w[i], exact) == kPairsPass;
+  const int from = !pairs_by_chunks(G, evaluated, exact) ? kPairsPass + 1 : sums_join_pairs(G) ? kSumsPass : kPairsPass;
   WedgeSet rank = ws, pairs = ws;
   rank.np = pairs.np = 0;
   for (int i = 0; i < ws.np; i++) {
-    WedgeSet& to = wedge_pass(G, ws.w[i]) >= from ? pairs : rank;
+    WedgeSet& to = wedge_pass(G, ws.w[i], exact) >= from ? pairs : rank;
     to.w[to.np] = ws.w[i];
     to.slot[to.np++] = ws.slot[i];
   }
@@ -1970,7 +1970,7 @@ int launch_wedge_set(DevGraph& G, const GView& gv, const WedgeSet& ws, cudaStrea
   const size_t arena = wedge_rank_scratch(G);
   if (arena > 0) st = ensure_plain_scratch(work.tri, std::max(arena, work.tri.bytes), s);
   if (st != FSGC_OK) return st;
-  st = enqueue_wedge_rank(G, gv, rank.w, rank.slot, rank.np, std::is_same<A, X128>::value, s, launches, work);
+  st = enqueue_wedge_rank(G, gv, rank.w, rank.slot, rank.np, exact, s, launches, work);
   return st == FSGC_EUNSUPPORTED ? launch_wedge_chunks<NP, A>(G, gv, rank, s, launches, work) : st;
 }
 

@@ -211,10 +211,10 @@ void free_rank_order(DevGraph& G);  // no work that reads it in flight
 // What a pattern's residual takes there: nothing of its own (none, or the pass over
 // the 4-cycles), a pass with sums per owner, or one that evaluates wedge() per pair.
 enum WedgePass { kNoPass = 0, kSumsPass = 1, kPairsPass = 2 };
-WedgePass wedge_pass(const DevGraph& G, const WedgeParams& p);
+WedgePass wedge_pass(const DevGraph& G, const WedgeParams& p, bool exact);
 // Whether `count` patterns of the last kind on an ordinary graph are better counted by
 // chunks, in one pass, and whether those with sums then join them.
-bool pairs_by_chunks(const DevGraph& G, int count);
+bool pairs_by_chunks(const DevGraph& G, int count, bool exact);
 bool sums_join_pairs(const DevGraph& G);
 int enqueue_wedge_rank(DevGraph& G, const GView& gv, const WedgeParams* pats, u64* const* slots, int np, bool exact,
                        cudaStream_t s, uint64_t* launches, DevWork& work);

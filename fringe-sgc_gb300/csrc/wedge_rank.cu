@@ -1306,9 +1306,9 @@ bool binomials_fit(int maxdeg, int k) {
   return k <= 2 || k * std::log2((double)std::max(2, maxdeg)) - std::lgamma((double)k) / std::log(2.0) < 63.0;
 }
 
-WedgePass wedge_pass(const DevGraph& G, const WedgeParams& p) {
+WedgePass wedge_pass(const DevGraph& G, const WedgeParams& p, bool exact) {
   long long mult = 0;
-  const bool fits = pattern_fits(G, p);
+  const bool fits = exact || pattern_fits(G, p);
   if (counts_four_cycles(p, &mult) || (fits && p.f_vw == 0 && std::min(p.f_v, p.f_w) == 0)) return kNoPass;
   return pair_form(p, fits).kind == kGeneral ? kPairsPass : kSumsPass;
 }
@@ -1327,10 +1327,12 @@ static double wedges_per_pair(const DevGraph& G) { return (double)G.m * G.mean_e
 //   RMAT n = 4,096, R = 1.1, S = 8: 0.31 0.28; 0.42 0.44; 1.10 1.31
 //   RMAT n = 16,384, R = 0.6, S = 14: 1.4 1.1; 1.9 1.6; 5.8 5.0
 //   cliques of 600 and 1,200, R = n - 1: 0.39 0.26, 2.3 1.1; 0.40 0.29, 2.3 1.2; 0.47 1.03, 2.5 4.5
-bool pairs_by_chunks(const DevGraph& G, int count) {
+// Exact counts, one pattern each: uniform, n = 600, R = 4: 0.14 0.37; 0.23 0.70   clique of
+// 300: 0.12 0.18; 0.13 0.24   RMAT n = 4,096, 52,000 entries, S = 8: 0.44 0.42; 0.64 0.70
+bool pairs_by_chunks(const DevGraph& G, int count, bool exact) {
   if (count == 0 || G.ngraphs > 0 || G.m == 0) return false;
   const double R = wedges_per_pair(G), S = G.mean_end_degree * (double)G.n / (double)G.m;
-  return count == 1 ? R >= 0.25 && R <= 256 && S <= 6.5 : R >= 0.08 && S <= 9;
+  return count == 1 ? R >= 0.25 && R <= (exact ? 512 : 256) && S <= 6.5 : R >= 0.08 && S <= 9;
 }
 
 // From about 16 wedges a pair of ids (the set above, its fourth pattern in rank order and
