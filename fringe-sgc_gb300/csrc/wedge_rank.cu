@@ -126,22 +126,11 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool same = f_v == f_w;
   A total = A(0);
-  auto span = [&](const int* nb, int d, int first, int stride, A& p_sum, A& q_sum, A& acc) {
-    for (int t0 = first; t0 < d; t0 += 4 * stride) {
-      int x[4], dx[4];  // four entries and their degrees in flight
-#pragma unroll
-      for (int k = 0; k < 4; k++) x[k] = d - t0 > k * stride ? __ldg(nb + t0 + k * stride) : -1;
-#pragma unroll
-      for (int k = 0; k < 4; k++) dx[k] = x[k] >= 0 ? __ldg(g.deg + x[k]) - 1 : 0;
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        if (x[k] < 0) break;
-        const A p = nck_a<A>(dx[k], f_v), q = same ? p : nck_a<A>(dx[k], f_w);
-        acc += same ? p * p_sum : p * q_sum + q * p_sum;
-        p_sum += p;
-        q_sum += q;
-      }
-    }
+  auto take = [&](int dx, A& p_sum, A& q_sum, A& acc) {
+    const A p = nck_a<A>(dx, f_v), q = same ? p : nck_a<A>(dx, f_w);
+    acc += same ? p * p_sum : p * q_sum + q * p_sum;
+    p_sum += p;
+    q_sum += q;
   };
   // consecutive vertices go to different blocks: hubs are often neighbours by id
   const int step = gridDim.x * (kTPB / 32);
@@ -152,7 +141,8 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
     A acc = A(0);
     if (d >= 2 && d <= kLinBlock) {
       A p = A(0), q = A(0);
-      span(g.adj + g.off[v], d, lane, 32, p, q, acc);
+      const int* nb = g.adj + g.off[v];
+      for (int t = lane; t < d; t += 32) take(g.deg[__ldg(nb + t)] - 1, p, q, acc);
       const A pe = warp_excl(p), qe = same ? pe : warp_excl(q);
       acc += same ? p * pe : p * qe + q * pe;
     }
@@ -168,7 +158,18 @@ __global__ void __launch_bounds__(kTPB) wedge_linear_kernel(GView g, int f_v, in
       const int h = s_big[b];
       if (h < 0) continue;
       A p = A(0), q = A(0), a2 = A(0);
-      span(g.adj + g.off[h], g.deg[h], threadIdx.x, kTPB, p, q, a2);
+      const int* nb = g.adj + g.off[h];
+      const int dh = g.deg[h];
+      for (int t0 = threadIdx.x; t0 < dh; t0 += 4 * kTPB) {
+        int x[4], dx[4];  // four entries and their degrees in flight
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = t0 + k * kTPB < dh ? __ldg(nb + t0 + k * kTPB) : -1;
+#pragma unroll
+        for (int k = 0; k < 4; k++) dx[k] = x[k] >= 0 ? __ldg(g.deg + x[k]) - 1 : 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (x[k] >= 0) take(dx[k], p, q, a2);
+      }
       const A pe = warp_excl(p), qe = same ? pe : warp_excl(q);
       a2 += same ? p * pe : p * qe + q * pe;
       if (lane == 31) {
