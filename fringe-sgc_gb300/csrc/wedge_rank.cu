@@ -779,9 +779,9 @@ __device__ __noinline__ A scan_general(const RankView& r, const RankSet& rs, Ran
 // an instruction), dependent instructions (2.1, 2.3) and barriers (1.8, 2.5); the
 // shared-memory adds, 2.9 cycles a warp and SM where they are random, are 13 and 12 %
 // of the time, DRAM 6 and 1.5 % of its rate.  Whole counts there, before -> after, with
-// the linear pass (1.4 to 2.4 ms) and the adjacent one (0.3 to 1.1 ms): one fringe on
-// each end 344 -> 17 ms (ORD), 4-cycle with opposite fringes 327 -> 87 ms, three
-// fringes and one 636 -> 98 ms.  The copy in rank order is built once per graph: 5 ms.
+// the linear pass (2.3 to 3.2 ms) and the adjacent one (0.3 to 1.1 ms): one fringe on
+// each end 344 -> 18 ms (ORD), 4-cycle with opposite fringes 327 -> 87 ms, three
+// fringes and one 636 -> 99 ms.  The copy in rank order is built once per graph: 5 ms.
 template <bool ORD, class A>
 __global__ void __launch_bounds__(kRT, 2) wedge_rank_kernel(const __grid_constant__ RankView r,
                                                             const __grid_constant__ RankSet rs,
